@@ -130,26 +130,43 @@ static size_t elem_bytes_h(int prec) { return prec == WTD_MIXED_H32 ? sizeof(flo
 /* ---------------------------------------------------------------------------------------
  * fused pass dispatch
  * -------------------------------------------------------------------------------------*/
-template <typename TC, int NBUF> static constexpr size_t fused_smem() { return FusedSmem<WG, TC, NBUF>::bytes; }
+/* the fused pass of one form: its kernel, threads per CTA and shared memory.  WTD_BLOCK=1024
+ * selects 1024-thread CTAs for the transforms' form on lattices of at least 2048 points; the
+ * folded-line form has the one block size of FusedCfg */
+template <typename TY, typename TH, typename TC, int PASS, bool GRAD> struct FusedLaunch {
+    typedef FusedCfg<WG, TC, WTD_VAR> Cfg;
+    static constexpr size_t smem = FusedSmem<WG, TC, WTD_VAR, GRAD>::bytes;
+    static constexpr bool fits = smem <= WTD_SMEM_MAX && FusedSmem<WG, TC, WTD_VAR, GRAD>::fft_bytes <= WTD_SMEM_MAX;
+    static constexpr bool wide = !Cfg::circ && WG::ntot >= 2048;
+    template <int BS> static auto kernel()
+    {
+        return wtd_fused_pass<WG, TY, TH, TC, WTD_NHIST, PASS, WTD_VAR, GRAD, BS,
+                              Cfg::circ || BS == 512 ? Cfg::minb : 1>;
+    }
+    static constexpr int BS = Cfg::circ ? Cfg::threads : 512;
+};
 
 template <typename TY, typename TH, typename TC, int PASS, bool GRAD>
 static int launch_pass_t(wtd_ctx *c, StepArgs &a)
 {
-    constexpr int NBUF = WTD_VAR ? 4 : (GRAD ? 3 : 2);
-    constexpr size_t sm = fused_smem<TC, NBUF>();
-    if (sm > WTD_SMEM_MAX) return WTD_ERR_UNSUPPORTED;
+    typedef FusedLaunch<TY, TH, TC, PASS, GRAD> L;
+    if constexpr (!L::fits) return WTD_ERR_UNSUPPORTED;
     else {
-        if (c->block == 1024 && WG::ntot >= 2048) {
-            auto k = wtd_fused_pass<WG, TY, TH, TC, WTD_NHIST, PASS, WTD_VAR, GRAD, 1024>;
+        bool done = false;
+        if constexpr (L::wide) {
+            if (c->block == 1024) {
+                auto k = L::template kernel<1024>();
+                WTD_ONCE_PER_DEVICE(
+                    WTD_CU(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L::smem)));
+                k<<<c->grid, 1024, L::smem, c->st>>>(a, c->tw, c->ktab);
+                done = true;
+            }
+        }
+        if (!done) {
+            auto k = L::template kernel<L::BS>();
             WTD_ONCE_PER_DEVICE(
-                WTD_CU(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm)));
-            k<<<c->grid, 1024, sm, c->st>>>(a, c->tw, c->ktab);
-        } else {
-            auto k = wtd_fused_pass<WG, TY, TH, TC, WTD_NHIST, PASS, WTD_VAR, GRAD, 512>;
-            WTD_ONCE_PER_DEVICE(
-                WTD_CU(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm)));
-            int threads = WG::ntot >= 512 ? 512 : ((WG::ntot + 31) / 32) * 32;
-            k<<<c->grid, threads, sm, c->st>>>(a, c->tw, c->ktab);
+                WTD_CU(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L::smem)));
+            k<<<c->grid, L::Cfg::threads, L::smem, c->st>>>(a, c->tw, c->ktab);
         }
         WTD_LAUNCHED(c);
     }
@@ -842,22 +859,27 @@ static int occupancy_t(int block)
 {
     /* resident CTAs of the step's ordinary passes (PASS 0 without gradients); the gradient
      * passes (one more buffer) may then run the same grid in more than one wave */
-    constexpr int NBUF = WTD_VAR ? 4 : 2;
-    constexpr size_t sm = fused_smem<TC, NBUF>();
-    if (sm > WTD_SMEM_MAX) return 1;
-    int nb = 1;
-    if (block == 1024 && WG::ntot >= 2048) {
-        auto k = wtd_fused_pass<WG, TY, TH, TC, WTD_NHIST, 0, WTD_VAR, false, 1024>;
-        cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k, 1024, sm);
-    } else {
-        auto k = wtd_fused_pass<WG, TY, TH, TC, WTD_NHIST, 0, WTD_VAR, false, 512>;
-        cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-        int threads = WG::ntot >= 512 ? 512 : ((WG::ntot + 31) / 32) * 32;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k, threads, sm);
+    typedef FusedLaunch<TY, TH, TC, 0, false> L;
+    if constexpr (!L::fits) return 1;
+    else {
+        int nb = 1;
+        bool done = false;
+        if constexpr (L::wide) {
+            if (block == 1024) {
+                auto k = L::template kernel<1024>();
+                cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L::smem);
+                cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k, 1024, L::smem);
+                done = true;
+            }
+        }
+        if (!done) {
+            auto k = L::template kernel<L::BS>();
+            cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L::smem);
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k, L::Cfg::threads, L::smem);
+        }
+        cudaGetLastError();
+        return nb < 1 ? 1 : (nb > 16 ? 16 : nb);
     }
-    cudaGetLastError();
-    return nb < 1 ? 1 : (nb > 16 ? 16 : nb);
 }
 
 static int occupancy_per_sm(wtd_ctx *c)

@@ -31,6 +31,7 @@
 #define WTD_STEP_CUH
 
 #include "wtd_core.cuh"
+#include "wtd_circ.cuh"
 
 /* per-point coefficients prepared once per half-step from the potentials */
 enum {
@@ -143,11 +144,39 @@ __device__ __forceinline__ void kmul(C *buf, const double (*kt)[WTD_KT])
 /* ---------------------------------------------------------------------------------------
  * shared-memory layout of the fused kernel
  * -------------------------------------------------------------------------------------*/
-template <class G, typename TC, int NBUF> struct FusedSmem {
+/* the fused kernel's form on a lattice: folded circulant lines (wtd_circ.cuh) where they fit, else
+ * the transforms of wtd_core.cuh */
+template <class G, typename TC, bool VAR> struct FusedCfg {
+    typedef CircGeo<G> CG;
+    /* FP64 lines of more than 48 points need 255 registers, which leaves 256 threads an SM: the
+     * laplacian is faster all the same (64^2: 4.6 us a field against 6.6 us) but pass A's streaming
+     * phases, which live on loads in flight, lose more (8192 states: 2.74 ms against 2.15 ms) */
+    static constexpr bool circ = CG::fits && (sizeof(TC) == 4 || CG::nmax <= 48);
+    typedef typename std::conditional<circ, CG, G>::type Lay;   /* layout of a field in shared memory */
+    /* threads.  Lines of more than 32 points take 128 to 255 registers in FP64, so such lattices
+     * run as many threads as they have lines (at most 256), and all lines are in registers at
+     * once; the others run 256 threads */
+    static constexpr int lines = (CG::total + 31) / 32 * 32;
+    static constexpr int pts = (G::ntot + 31) / 32 * 32;
+    static constexpr int threads = !circ ? (G::ntot >= 512 ? 512 : pts)
+                                 : CG::nmax > 32 ? (lines < 128 ? 128 : lines > 256 ? 256 : lines)
+                                 : pts < 256 ? (pts > lines ? pts : lines > 256 ? 256 : lines) : 256;
+    /* CTAs per SM asked of the register allocator */
+    static constexpr int minb = !circ ? (sizeof(TC) == 4 && threads == 512 ? 2 : 1)
+                              : CG::nmax > (sizeof(TC) == 4 ? 64 : 48) || (VAR && CG::nmax > 16) ? 1 : 2;
+    static constexpr bool inplace = circ && !VAR && CG::total <= threads;
+    static constexpr int nbuf(bool grad) { return !circ ? (VAR ? 4 : grad ? 3 : 2) : inplace && !grad ? 2 : 3; }
+};
+
+template <class G, typename TC, bool VAR, bool GRAD> struct FusedSmem {
     typedef typename cplx<TC>::t C;
-    static constexpr size_t buf_bytes = (size_t)G::padded * sizeof(C);
-    static constexpr size_t tw_bytes = (size_t)G::twtotal * sizeof(C);
-    static constexpr size_t bytes = NBUF * buf_bytes + tw_bytes + sizeof(KTab<G>) + 80 * sizeof(double);
+    typedef FusedCfg<G, TC, VAR> Cfg;
+    static constexpr size_t buf_bytes = (size_t)Cfg::Lay::padded * sizeof(C);
+    static constexpr size_t tab_bytes = Cfg::circ ? 0 : (size_t)G::twtotal * sizeof(C) + sizeof(KTab<G>);
+    static constexpr size_t bytes = Cfg::nbuf(GRAD) * buf_bytes + tab_bytes + 80 * sizeof(double);
+    /* what the transforms' layout needs: lattices beyond it are refused in either form */
+    static constexpr size_t fft_bytes = (size_t)(VAR ? 4 : GRAD ? 3 : 2) * G::padded * sizeof(C) +
+                                        (size_t)G::twtotal * sizeof(C) + sizeof(KTab<G>) + 80 * sizeof(double);
 };
 
 /* load twiddles (e^{-2 pi i t/n} per axis) and the k tables into shared memory */
@@ -168,30 +197,51 @@ __device__ __forceinline__ void load_tables(C *tw, double (*kt)[WTD_KT], const d
  * On return BU/BV hold (H psi) in natural order (compute precision) and the function returns
  * <psi|H|psi> dV.  pca_kernels.cu:233-391 (const-mass branches) and :393-495 (BdG).
  * -------------------------------------------------------------------------------------*/
-template <class G, typename TY, typename TC>
+template <class Cfg, class G, typename TY, typename TC>
 __device__ __forceinline__ double hpsi_const(const TY *yu, const TY *yv, typename cplx<TC>::t *BU,
-                                             typename cplx<TC>::t *BV, const typename cplx<TC>::t *tw,
-                                             const double (*kt)[WTD_KT], const double *cf, double kp2, double *red)
+                                             typename cplx<TC>::t *BV, typename cplx<TC>::t *B2,
+                                             const typename cplx<TC>::t *tw, const double (*kt)[WTD_KT], const double *cf,
+                                             double kp2, double *red)
 {
     typedef typename cplx<TC>::t C;
+    typedef typename Cfg::Lay Lay;
     constexpr int N = G::ntot;
     const uint64_t pol = l2_policy_keep();
-    for (int p = threadIdx.x; p < N; p += blockDim.x) {
-        double2 u = to_d(yu[p]), v = to_d(yv[p]);
-        int o = G::off(p);
-        BU[o].x = (TC)u.x; BU[o].y = (TC)u.y;
-        BV[o].x = (TC)v.x; BV[o].y = (TC)v.y;
+    if constexpr (Cfg::circ && !Cfg::inplace) {
+#pragma unroll 1
+        for (int comp = 0; comp < 2; comp++) {
+            const TY *y = comp ? yv : yu;
+            for (int p = threadIdx.x; p < N; p += blockDim.x) {
+                const double2 a = to_d(y[p]);
+                C z; z.x = (TC)a.x; z.y = (TC)a.y;
+                B2[Lay::off(p)] = z;
+            }
+            __syncthreads();
+            circ_lap<Lay, false>(B2, comp ? BV : BU);
+        }
+    } else {
+        for (int p = threadIdx.x; p < N; p += blockDim.x) {
+            double2 u = to_d(yu[p]), v = to_d(yv[p]);
+            int o = Lay::off(p);
+            BU[o].x = (TC)u.x; BU[o].y = (TC)u.y;
+            BV[o].x = (TC)v.x; BV[o].y = (TC)v.y;
+        }
+        __syncthreads();
+        if constexpr (Cfg::circ) {
+#pragma unroll 1
+            for (int comp = 0; comp < 2; comp++) circ_lap<Lay, true>(comp ? BV : BU, comp ? BV : BU);
+        } else {
+            fft_forward<G, 2>(BU, (int)(BV - BU), tw);
+            kmul<G, OP_LAP>(BU, kt);
+            kmul<G, OP_LAP>(BV, kt);
+            __syncthreads();
+            fft_inverse<G, 2>(BU, (int)(BV - BU), tw);
+        }
     }
-    __syncthreads();
-    fft_forward<G, 2>(BU, (int)(BV - BU), tw);
-    kmul<G, OP_LAP>(BU, kt);
-    kmul<G, OP_LAP>(BV, kt);
-    __syncthreads();
-    fft_inverse<G, 2>(BU, (int)(BV - BU), tw);
     double q = 0.0;
 #pragma unroll 2
     for (int p = threadIdx.x; p < N; p += blockDim.x) {
-        int o = G::off(p);
+        int o = Lay::off(p);
         TC ur, ui, vr, vi;
         {
             double2 u = to_d(yu[p]), v = to_d(yv[p]);
@@ -223,17 +273,18 @@ __device__ __forceinline__ double hpsi_const(const TY *yu, const TY *yv, typenam
  *        + (1/4) alpha_b lap v + (1/4) lap(alpha_b v)
  * Buffers: B0 (transform of one component), W (work), HU, HV (results).
  * -------------------------------------------------------------------------------------*/
-template <class G, typename TY, typename TC>
+template <class Cfg, class G, typename TY, typename TC>
 __device__ __forceinline__ double hpsi_var(const TY *yu, const TY *yv, typename cplx<TC>::t *B0,
                                            typename cplx<TC>::t *W, typename cplx<TC>::t *HU,
                                            typename cplx<TC>::t *HV, const typename cplx<TC>::t *tw,
                                            const double (*kt)[WTD_KT], const double *cf, double kp2, double *red)
 {
     typedef typename cplx<TC>::t C;
+    typedef typename Cfg::Lay Lay;
     constexpr int N = G::ntot;
     /* local terms into HU/HV */
     for (int p = threadIdx.x; p < N; p += blockDim.x) {
-        int o = G::off(p);
+        int o = Lay::off(p);
         double2 u = to_d(yu[p]), v = to_d(yv[p]);
         double va = cf[CF_VA * N + p], vb = cf[CF_VB * N + p];
         double dr = cf[CF_DRE * N + p], di = cf[CF_DIM * N + p];
@@ -251,6 +302,54 @@ __device__ __forceinline__ double hpsi_var(const TY *yu, const TY *yv, typename 
         HU[o].x = (TC)hu.x; HU[o].y = (TC)hu.y;
         HV[o].x = (TC)hv.x; HV[o].y = (TC)hv.y;
     }
+    if constexpr (Cfg::circ) {
+#pragma unroll 1
+        for (int comp = 0; comp < 2; comp++) {
+            __syncthreads();
+            for (int p = threadIdx.x; p < N; p += blockDim.x) {
+                const double2 a = to_d((comp ? yv : yu)[p]);
+                C z; z.x = (TC)a.x; z.y = (TC)a.y;
+                B0[Lay::off(p)] = z;
+            }
+            __syncthreads();
+            const TC s4 = comp ? (TC)0.25 : (TC)-0.25;
+            const double *al = cf + (size_t)(CF_ALA + comp) * N, *A = cf + (size_t)(comp ? CF_ABX : CF_AAX) * N;
+            const TC *s = (const TC *)B0;
+#pragma unroll 1
+            for (int r0 = 0; r0 < Lay::total; r0 += blockDim.x) {
+                const CircLine<Lay> L(r0 + threadIdx.x);
+                TC own[Lay::nmax], crs[Lay::nmax];
+#pragma unroll
+                for (int j = 0; j < Lay::nmax; j++) own[j] = crs[j] = (TC)0;
+                if (L.on)
+                    circ_axis<Lay>(L.ax, [&](auto AXC) {
+                        constexpr int AX = decltype(AXC)::value, n = Lay::n(AX);
+                        const double *Aa = A + (size_t)L.ax * N;
+                        TC l[n];
+                        circ::MemLine<TC> f{s + L.base, L.st};
+                        /* -i A d psi: the re line adds to im, the im line to re */
+                        circ::line_from<circ::DER, AX, n>(f, l);
+#pragma unroll
+                        for (int j = 0; j < n; j++) crs[j] = (L.c ? (TC)1 : (TC)-1) * (TC)Aa[L.pb + j * L.ps] * l[j];
+                        /* -1/4 (alpha lap psi + lap(alpha psi)) with the spin's sign */
+                        circ::line_from<circ::LAP, AX, n>(f, l);
+                        TC g[n];
+#pragma unroll
+                        for (int j = 0; j < n; j++) {
+                            const TC a = (TC)al[L.pb + j * L.ps];
+                            own[j] = s4 * a * l[j];
+                            g[j] = a * f(j);
+                        }
+                        circ::line_op<circ::LAP, AX, n>(g, l);
+#pragma unroll
+                        for (int j = 0; j < n; j++) own[j] += s4 * l[j];
+                    });
+#pragma unroll
+                for (int j = 0; j < Lay::nmax; j++) own[j] += __shfl_xor_sync(0xffffffffu, crs[j], 1);
+                circ_store<Lay, true>((TC *)(comp ? HV : HU), L, own, r0);
+            }
+        }
+    } else
     for (int comp = 0; comp < 2; comp++) {
         const TY *y = comp == 0 ? yu : yv;
         C *H = comp == 0 ? HU : HV;
@@ -314,7 +413,7 @@ __device__ __forceinline__ double hpsi_var(const TY *yu, const TY *yv, typename 
     __syncthreads();
     double q = 0.0;
     for (int p = threadIdx.x; p < N; p += blockDim.x) {
-        int o = G::off(p);
+        int o = Lay::off(p);
         double2 u = to_d(yu[p]), v = to_d(yv[p]);
         C hu = HU[o], hv = HV[o];
         q += u.x * (double)hu.x + u.y * (double)hu.y + v.x * (double)hv.x + v.y * (double)hv.y;
@@ -354,7 +453,7 @@ __device__ __forceinline__ void dens_limited_red(double *ds, int p, int N, doubl
  * component in natural order and is transformed in place; W is work; ysrc gives the stored
  * normalised values.  tau_tmp_s += f_s Re(conj(psi)(lap psi - |k_perp|^2 psi)),
  * j_s,d += (+1 for u, -1 for v) f_s Im(conj(psi) d_d psi). */
-template <class G, typename TY, typename TC>
+template <class Cfg, class G, typename TY, typename TC>
 __device__ __forceinline__ void dens_gradients(double *ds, const TY *ysrc, typename cplx<TC>::t *B0,
                                                typename cplx<TC>::t *W, const typename cplx<TC>::t *tw,
                                                const double (*kt)[WTD_KT], double f, double w, double kp2, int comp,
@@ -371,44 +470,85 @@ __device__ __forceinline__ void dens_gradients(double *ds, const TY *ysrc, typen
     const double jsgn = comp == 0 ? 1.0 : -1.0;
     /* slot updates as L2 reductions: each word of the CTA's slot is updated by one thread only */
     const uint64_t pol = l2_policy_keep();
-    __syncthreads();
-    fft_forward<G, 1>(B0, 0, tw);
-    for (int op = 0; op <= G::dims; op++) {
-        for (int i = threadIdx.x; i < G::padded; i += blockDim.x) W[i] = B0[i];
-        __syncthreads();
-        if (op == 0) kmul<G, OP_LAP>(W, kt);
-        else if (op == 1) kmul<G, OP_DX>(W, kt);
-        else if (op == 2) kmul<G, OP_DY>(W, kt);
-        else kmul<G, OP_DZ>(W, kt);
-        __syncthreads();
-        fft_inverse<G, 1>(W, 0, tw);
-        for (int p = threadIdx.x; p < N; p += blockDim.x) {
-            double2 sv = to_d(ysrc[p]);
-            C d = W[G::off(p)];
-            double dx = d.x, dy = d.y;
-            if (op == 0) {
-                double lx = dx - sv.x * kp2, ly = dy - sv.y * kp2;
-                red_keep(ds + tau_q * (size_t)N + p, (sv.x * lx + sv.y * ly) * fw, pol);
-                if (yother) {
-                    const double2 o = to_d(yother[p]);
-                    const double im = sv.x * ly - sv.y * lx; /* Im[psi* lap psi] */
-                    if (comp == 0) {
-                        red_keep(ds + 12 * (size_t)N + p, im * fw, pol);
-                        /* v* lap u */
-                        red_keep(ds + 14 * (size_t)N + 2 * p, (o.x * lx + o.y * ly) * fq, pol);
-                        red_keep(ds + 14 * (size_t)N + 2 * p + 1, (o.x * ly - o.y * lx) * fq, pol);
-                    } else {
-                        red_keep(ds + 13 * (size_t)N + p, -(im * fw), pol);
-                        /* (lap v)* u */
-                        red_keep(ds + 14 * (size_t)N + 2 * p, (lx * o.x + ly * o.y) * fq, pol);
-                        red_keep(ds + 14 * (size_t)N + 2 * p + 1, (lx * o.y - ly * o.x) * fq, pol);
-                    }
-                }
+    /* tau (and the friction densities) at point p from the laplacian d of the component there */
+    auto tau_point = [&](int p, double2 sv, double dx, double dy) {
+        double lx = dx - sv.x * kp2, ly = dy - sv.y * kp2;
+        red_keep(ds + tau_q * (size_t)N + p, (sv.x * lx + sv.y * ly) * fw, pol);
+        if (yother) {
+            const double2 o = to_d(yother[p]);
+            const double im = sv.x * ly - sv.y * lx; /* Im[psi* lap psi] */
+            if (comp == 0) {
+                red_keep(ds + 12 * (size_t)N + p, im * fw, pol);
+                /* v* lap u */
+                red_keep(ds + 14 * (size_t)N + 2 * p, (o.x * lx + o.y * ly) * fq, pol);
+                red_keep(ds + 14 * (size_t)N + 2 * p + 1, (o.x * ly - o.y * lx) * fq, pol);
             } else {
-                red_keep(ds + (j_q + op - 1) * (size_t)N + p, jsgn * (sv.x * dy - sv.y * dx) * fw, pol);
+                red_keep(ds + 13 * (size_t)N + p, -(im * fw), pol);
+                /* (lap v)* u */
+                red_keep(ds + 14 * (size_t)N + 2 * p, (lx * o.x + ly * o.y) * fq, pol);
+                red_keep(ds + 14 * (size_t)N + 2 * p + 1, (lx * o.y - ly * o.x) * fq, pol);
             }
         }
+    };
+    __syncthreads();
+    if constexpr (Cfg::circ) {
+        typedef typename Cfg::Lay Lay;
+        const TC *s = (const TC *)B0;
+        circ_lap<Lay, false>(B0, W);
+#pragma unroll 1
+        for (int r0 = 0; r0 < Lay::total; r0 += blockDim.x) {
+            const CircLine<Lay> L(r0 + threadIdx.x);
+            TC d[Lay::nmax];
+#pragma unroll
+            for (int j = 0; j < Lay::nmax; j++) d[j] = (TC)0;
+            if (L.on)
+                circ_axis<Lay>(L.ax, [&](auto AXC) {
+                    constexpr int AX = decltype(AXC)::value, n = Lay::n(AX);
+                    TC l[n];
+                    circ::MemLine<TC> f{s + L.base, L.st};
+                    circ::line_from<circ::DER, AX, n>(f, l);
+#pragma unroll
+                    for (int j = 0; j < n; j++) d[j] = l[j];
+                });
+            /* Im(psi* d psi) = re d im - im d re over the pair of lines; the re line's thread
+             * updates the slot, the same thread for every state */
+            double *dj = ds + (size_t)(j_q + L.ax) * N + L.pb;
+            const int nax = L.ax == 0 ? Lay::n(0) : L.ax == 1 ? Lay::n(1) : Lay::n(2);
+            int st = L.st;
+            asm volatile("" : "+r"(st));
+#pragma unroll
+            for (int j = 0; j < Lay::nmax; j++) {
+                const double o = j < nax ? (double)s[(L.base ^ 1) + j * st] : 0.0;
+                const double a = (L.c ? 1.0 : -1.0) * o * (double)d[j];
+                const double b = a + __shfl_xor_sync(0xffffffffu, a, 1);
+                if (L.on && L.c == 0 && j < nax) red_keep(dj + (size_t)j * L.ps, jsgn * b * fw, pol);
+            }
+        }
+        for (int p = threadIdx.x; p < N; p += blockDim.x) {
+            const C d = W[Lay::off(p)];
+            tau_point(p, to_d(ysrc[p]), (double)d.x, (double)d.y);
+        }
         __syncthreads();
+    } else {
+        fft_forward<G, 1>(B0, 0, tw);
+        for (int op = 0; op <= G::dims; op++) {
+            for (int i = threadIdx.x; i < G::padded; i += blockDim.x) W[i] = B0[i];
+            __syncthreads();
+            if (op == 0) kmul<G, OP_LAP>(W, kt);
+            else if (op == 1) kmul<G, OP_DX>(W, kt);
+            else if (op == 2) kmul<G, OP_DY>(W, kt);
+            else kmul<G, OP_DZ>(W, kt);
+            __syncthreads();
+            fft_inverse<G, 1>(W, 0, tw);
+            for (int p = threadIdx.x; p < N; p += blockDim.x) {
+                double2 sv = to_d(ysrc[p]);
+                C d = W[G::off(p)];
+                double dx = d.x, dy = d.y;
+                if (op == 0) tau_point(p, sv, dx, dy);
+                else red_keep(ds + (j_q + op - 1) * (size_t)N + p, jsgn * (sv.x * dy - sv.y * dx) * fw, pol);
+            }
+            __syncthreads();
+        }
     }
 }
 
@@ -421,30 +561,38 @@ __device__ __forceinline__ void dens_gradients(double *ds, const TY *ysrc, typen
  *               apply_hamiltonian into f1 (pca.c:1565), formed on demand
  * VAR: variable effective mass; GRAD: tau and j of the output state too.
  * -------------------------------------------------------------------------------------*/
-template <class G, typename TY, typename TH, typename TC, int NH, int PASS, bool VAR, bool GRAD, int BS>
-__global__ void __launch_bounds__(BS, (sizeof(TC) == 4 && BS == 512) ? 2 : 1) /* FP32 compute: 2 CTAs/SM */
+template <class G, typename TY, typename TH, typename TC, int NH, int PASS, bool VAR, bool GRAD, int BS, int MINB>
+__global__ void __launch_bounds__(BS, MINB)
 wtd_fused_pass(StepArgs a, const double2 *gtw, const double *gk)
 {
     typedef typename cplx<TC>::t C;
+    typedef FusedCfg<G, TC, VAR> Cfg;
+    typedef typename Cfg::Lay Lay;
     constexpr int N = G::ntot;
-    constexpr int NBUF = VAR ? 4 : (GRAD ? 3 : 2);
+    constexpr int NBUF = Cfg::nbuf(GRAD);
     extern __shared__ __align__(16) unsigned char smem_raw[];
     C *BU = (C *)smem_raw;
-    C *BV = BU + G::padded;
-    C *B2 = BV + G::padded;
-    C *B3 = B2 + G::padded;
-    C *tw = BU + NBUF * G::padded;
+    C *BV = BU + Lay::padded;
+    C *B2 = BV + Lay::padded;
+    C *tw = BU + NBUF * Lay::padded;
     double (*kt)[WTD_KT] = (double (*)[WTD_KT])(tw + G::twtotal);
-    double *red = (double *)(kt + 6);
+    double *red = Cfg::circ ? (double *)tw : (double *)(kt + 6);
 
-    load_tables<G>(tw, kt, gtw, gk);
+    if constexpr (!Cfg::circ) load_tables<G>(tw, kt, gtw, gk);
 
     TY *Y = (TY *)a.y;
     TY *YO = a.yout ? (TY *)a.yout : Y;
     const uint64_t pol = l2_policy_keep();
     double *ds = a.dslot + (size_t)blockIdx.x * a.sstride;
-    if (!a.accumulate)
-        for (int i = threadIdx.x; i < a.sstride; i += blockDim.x) ds[i] = 0.0;
+    if (!a.accumulate) {
+        /* without gradients the slot holds nu, rho_a and rho_b only */
+        if (GRAD || PASS == 3) {
+            for (int i = threadIdx.x; i < a.sstride; i += blockDim.x) ds[i] = 0.0;
+        } else {
+            for (int i = threadIdx.x; i < 3 * N; i += blockDim.x) ds[i] = 0.0;
+            for (int i = threadIdx.x; i < N; i += blockDim.x) ds[7 * (size_t)N + i] = 0.0;
+        }
+    }
     const double dt = a.dt;
     const size_t SN = (size_t)a.S * N;
 
@@ -480,16 +628,16 @@ wtd_fused_pass(StepArgs a, const double2 *gtw, const double *gk)
             }
         }
         /* results of H land in (HU, HV) */
-        C *HU = VAR ? B2 : BU, *HV = VAR ? B3 : BV;
+        C *HU = !VAR ? BU : Cfg::circ ? BV : B2, *HV = !VAR ? BV : Cfg::circ ? B2 : B2 + Lay::padded;
         double E = 0.0;
         if (haveH) {
-            if (VAR) E = hpsi_var<G, TY, TC>(yu, yv, BU, BV, HU, HV, tw, kt, a.cf, kp2, red);
-            else E = hpsi_const<G, TY, TC>(yu, yv, BU, BV, tw, kt, a.cf, kp2, red);
+            if constexpr (VAR) E = hpsi_var<Cfg, G, TY, TC>(yu, yv, BU, BV, HU, HV, tw, kt, a.cf, kp2, red);
+            else E = hpsi_const<Cfg, G, TY, TC>(yu, yv, BU, BV, B2, tw, kt, a.cf, kp2, red);
             if (threadIdx.x == 0) a.qpe[n] = E;
         }
         if (PASS == 3) {
             for (int p = threadIdx.x; p < N; p += blockDim.x) {
-                const int o = G::off(p);
+                const int o = Lay::off(p);
 #pragma unroll
                 for (int comp = 0; comp < 2; comp++) {
                     const size_t gi = (comp ? SN : 0) + (size_t)n * N + p;
@@ -510,7 +658,7 @@ wtd_fused_pass(StepArgs a, const double2 *gtw, const double *gk)
         double nrm = 0.0;
 #pragma unroll 2
         for (int p = threadIdx.x; p < N; p += blockDim.x) {
-            const int o = G::off(p);
+            const int o = Lay::off(p);
             /* all global loads of this point first (both components), then arithmetic */
             double2 y0[2], fr[2][NR > 0 ? NR : 1], fkg[2];
 #pragma unroll
@@ -583,7 +731,7 @@ wtd_fused_pass(StepArgs a, const double2 *gtw, const double *gk)
 #pragma unroll
             for (int k = 0; k < 2; k++) {
                 if (k == 1 && !hq) { uu[1] = vv[1] = make_double2(0.0, 0.0); break; }
-                const int pp = k ? q : p, o = G::off(pp);
+                const int pp = k ? q : p, o = Lay::off(pp);
                 C hu = HU[o], hv = HV[o];
                 double2 u = make_double2((double)hu.x * c, (double)hu.y * c);
                 double2 v = make_double2((double)hv.x * c, (double)hv.y * c);
@@ -604,8 +752,11 @@ wtd_fused_pass(StepArgs a, const double2 *gtw, const double *gk)
             /* const mass: (HU, HV) = (BU, BV) hold the state, B2 is work.
              * variable mass: (HU, HV) = (B2, B3), BU is work. */
             C *Wk = VAR ? BU : B2;
-            dens_gradients<G, TY, TC>(ds, ou, HU, Wk, tw, kt, f, w, kp2, 0, a.qf ? ov : nullptr);
-            dens_gradients<G, TY, TC>(ds, ov, HV, Wk, tw, kt, f, w, kp2, 1, a.qf ? ou : nullptr);
+            /* one instance of the line operators for both components */
+#pragma unroll 1
+            for (int comp = 0; comp < 2; comp++)
+                dens_gradients<Cfg, G, TY, TC>(ds, comp ? ov : ou, comp ? HV : HU, Wk, tw, kt, f, w, kp2, comp,
+                                               a.qf ? (comp ? ou : ov) : nullptr);
         }
         __syncthreads();
     }

@@ -52,6 +52,11 @@ struct wtd_ctx {
     int ncl;                    /* clusters of the x-line kernel */
     int g2;                     /* state chunks of the plane density kernel */
     int p1grid;                 /* CTAs of the plane H kernel */
+    /* stream path (wtd_stream3d.cuh), the form of the line path on axes of at most 64 points */
+    int stream;
+    double *sc, *part;          /* scale 1/norm of every state; partial sums of <H> and the norm */
+    int xgrid;                  /* CTAs of the x kernel */
+    int gpt, gpl, gx;           /* state chunks of the point, plane and x density kernels */
     void *xfer;                 /* bounded staging buffer of the mixed-precision uploads/downloads */
     /* state-sharded runs: sum of the density partials over ranks (NCCL or a host hook) */
     void *nccl;
@@ -220,6 +225,7 @@ static int run_pass(wtd_ctx *c, int pass, bool grad)
 }
 
 static int line_pass(wtd_ctx *c, int pass, bool grad, const StepArgs *given = NULL);
+static int stream_pass(wtd_ctx *c, int pass, bool grad);
 
 /* f1 = (H - <H>) psi of the current state and its quasiparticle energies, as the reference
  * leaves them after a step (pca.c:1565, d_workarea[0..n)); later steps reuse f1 */
@@ -227,7 +233,8 @@ static int ensure_fk(wtd_ctx *c)
 {
     if (c->fk_given) return WTD_OK;
     if (!c->have_coef) return WTD_ERR_STATE;
-    if (c->line) WTD_TRY(line_pass(c, 3, false));
+    if (c->stream) WTD_TRY(stream_pass(c, 3, false));
+    else if (c->line) WTD_TRY(line_pass(c, 3, false));
     else WTD_TRY(run_pass(c, 3, false));
     c->fk_given = 1;
     return WTD_OK;
@@ -555,6 +562,210 @@ static int staged_step(wtd_ctx *c, bool last)
     c->it++;
     return WTD_OK;
 }
+
+/* ---------------------------------------------------------------------------------------
+ * stream path (3D lattices beyond one CTA with axes of at most 64 points, wtd_stream3d.cuh)
+ * -------------------------------------------------------------------------------------*/
+#if CODEDIM == 3
+template <typename TC> struct StreamFit {
+    static constexpr bool ok = S3::ok && S3PlaneSmem<TC, WTD_VAR>::ok && S3XSmem<TC, WTD_VAR>::ok &&
+                               S3DensSmem<TC>::pbytes <= WTD_SMEM_MAX && S3DensSmem<TC>::xbytes <= WTD_SMEM_MAX;
+};
+static bool stream_fits(int prec)
+{
+    if (!WTD_BIG) return false;
+    return prec == WTD_FP64 ? StreamFit<double>::ok : StreamFit<float>::ok;
+}
+
+/* unnamed namespace: the statics of WTD_ONCE_PER_DEVICE inside a template with external linkage
+ * would be one object for all projects' libraries of a process */
+namespace {
+template <typename TY, typename TH, typename TC> struct Stream {
+    typedef typename cplx<TC>::t C;
+    typedef S3PlaneSmem<TC, WTD_VAR> PS;
+    typedef S3XSmem<TC, WTD_VAR> XS;
+    typedef S3DensSmem<TC> DS;
+
+    static int sum(wtd_ctx *c, int np, double *out, int norm, double *nrm_out = NULL)
+    {
+        k3s_sum<<<(c->S + 3) / 4, 128, 0, c->st>>>(c->part, np, c->S, out, norm, nrm_out);
+        WTD_LAUNCHED(c);
+        return WTD_OK;
+    }
+    template <int PASS> static int abm(wtd_ctx *c, const StepArgs &a)
+    {
+        k3s_abm<TY, TH, TC, WTD_NHIST, PASS><<<dim3(2 * S3::ACH, c->S), S3::AT, 0, c->st>>>(a, (const C *)c->kbuf, c->sc, c->part);
+        WTD_LAUNCHED(c);
+        return PASS == 3 ? WTD_OK : sum(c, 2 * S3::ACH, c->sc, 1);
+    }
+    static int attrs()
+    {
+        WTD_ONCE_PER_DEVICE(
+            WTD_CU(cudaFuncSetAttribute(k3s_plane_h<TY, TC, WTD_VAR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PS::bytes));
+            WTD_CU(cudaFuncSetAttribute(k3s_x_h<TY, TC, WTD_VAR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)XS::bytes));
+            WTD_CU(cudaFuncSetAttribute(k3s_dens_plane<TY, TC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DS::pbytes));
+            WTD_CU(cudaFuncSetAttribute(k3s_dens_x<TY, TC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DS::xbytes)));
+        return WTD_OK;
+    }
+    /* slots of the density kernels: points, planes, x lines */
+    static double *slots(wtd_ctx *c, int which)
+    {
+        constexpr size_t N = S3::N;
+        return c->dslot + (which > 0 ? (size_t)c->gpt * 4 * N : 0) + (which > 1 ? (size_t)c->gpl * 6 * N : 0);
+    }
+    static int pass(wtd_ctx *c, int p, bool grad)
+    {
+        const StepArgs a = make_args(c);
+        const TY *y = (const TY *)a.y;
+        if (p == 1 || p == 3 || (p == 0 && !a.fk_given)) {
+            k3s_plane_h<TY, TC, WTD_VAR><<<c->p1grid, S3::LT * PS::NS, PS::bytes, c->st>>>(y, (C *)c->kbuf, c->cf, c->sc, c->S);
+            WTD_LAUNCHED(c);
+            k3s_x_h<TY, TC, WTD_VAR><<<c->xgrid, 2 * S3::XL * XS::NS, XS::bytes, c->st>>>(y, (C *)c->kbuf, c->cf, c->sc, c->part, c->S);
+            WTD_LAUNCHED(c);
+            WTD_TRY(sum(c, 2 * S3::NQB, c->qpe, 0));
+        }
+        WTD_TRY(p == 0 ? abm<0>(c, a) : p == 1 ? abm<1>(c, a) : p == 2 ? abm<2>(c, a) : abm<3>(c, a));
+        if (p == 3) return WTD_OK;
+        constexpr int N = S3::N;
+        k3s_dens_points<TY><<<dim3((N + 127) / 128, c->gpt), 128, 0, c->st>>>(c->S, c->gpt, y, c->sc, c->occ, c->wcnt, slots(c, 0));
+        WTD_LAUNCHED(c);
+        if (grad) {
+            k3s_dens_plane<TY, TC><<<2 * NX * c->gpl, S3::LT, DS::pbytes, c->st>>>(c->S, c->gpl, y, c->sc, c->occ, c->wcnt, slots(c, 1));
+            WTD_LAUNCHED(c);
+            k3s_dens_x<TY, TC><<<S3::NQB * c->gx, 2 * S3::XL, DS::xbytes, c->st>>>(c->S, c->gx, y, c->sc, c->occ, c->wcnt, slots(c, 2));
+            WTD_LAUNCHED(c);
+        }
+        return WTD_OK;
+    }
+    static int rescale(wtd_ctx *c)
+    {
+        k3s_rescale<TY><<<dim3(2 * S3::ACH, c->S), S3::AT, 0, c->st>>>((TY *)c->y, c->sc, c->S);
+        WTD_LAUNCHED(c);
+        k3s_fill<<<(c->S + 255) / 256, 256, 0, c->st>>>(c->sc, 1.0, c->S);
+        WTD_LAUNCHED(c);
+        return WTD_OK;
+    }
+    /* CTAs of `unit` fixed pieces of work each split over chunks of states: about four rounds of
+     * the resident CTAs where that leaves each at least 8 iterations of `per` states, and never
+     * fewer than one round */
+    static int chunks(int nsm, int occ, int unit, int S, int per)
+    {
+        const int slots = nsm * (occ > 0 ? occ : 1), it = (S + per - 1) / per;
+        int n = (4 * slots + unit - 1) / unit;
+        if (n > it / 8) n = it / 8;
+        const int one = (slots + unit - 1) / unit;
+        if (n < one) n = one;
+        return n > it ? it : n < 1 ? 1 : n;
+    }
+    static int setup(wtd_ctx *c, int nsm)
+    {
+        WTD_TRY(attrs());
+        int o = 0;
+        WTD_CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, k3s_plane_h<TY, TC, WTD_VAR>, S3::LT * PS::NS, PS::bytes));
+        c->p1grid = 2 * NX * chunks(nsm, o, 2 * NX, c->S, PS::NS);
+        WTD_CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, k3s_x_h<TY, TC, WTD_VAR>, 2 * S3::XL * XS::NS, XS::bytes));
+        c->xgrid = S3::NQB * chunks(nsm, o, S3::NQB, c->S, XS::NS);
+        /* density slots are memory and a later sum: one round of resident CTAs */
+        auto one = [&](int occ, int unit) {
+            const int n = (nsm * (occ > 0 ? occ : 1) + unit - 1) / unit;
+            return n < 1 ? 1 : n > c->S ? c->S : n;
+        };
+        WTD_CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, k3s_dens_points<TY>, 128, 0));
+        c->gpt = one(o, (S3::N + 127) / 128);
+        WTD_CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, k3s_dens_plane<TY, TC>, S3::LT, DS::pbytes));
+        c->gpl = one(o, 2 * NX);
+        WTD_CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, k3s_dens_x<TY, TC>, 2 * S3::XL, DS::xbytes));
+        c->gx = one(o, S3::NQB);
+        return WTD_OK;
+    }
+};
+} // namespace
+
+/* f(Stream of the context's precision form) */
+template <class F> static int stream_form(wtd_ctx *c, F f)
+{
+    if (c->prec == WTD_FP64) {
+        if constexpr (WTD_BIG && StreamFit<double>::ok) return f(Stream<double2, double2, double>());
+    } else if constexpr (WTD_BIG && StreamFit<float>::ok) {
+        if (c->prec == WTD_MIXED_H64) return f(Stream<float2, double2, float>());
+        return f(Stream<float2, float2, float>());
+    }
+    return WTD_ERR_UNSUPPORTED;
+}
+static size_t stream_slot_words(const wtd_ctx *c) { return (size_t)(4 * c->gpt + 6 * c->gpl + 4 * c->gx) * S3::N; }
+static size_t stream_part_words(const wtd_ctx *c) { return (size_t)c->S * 2 * (S3::NQB > S3::ACH ? S3::NQB : S3::ACH); }
+
+/* one half step's kernels (pass 0: H y_k + predictor, 1: H y_pred + corrector, 2: norms and
+ * densities, 3: f_k only), timed like the fused passes when timing is on */
+static int stream_pass(wtd_ctx *c, int pass, bool grad)
+{
+    const bool timed = c->timing && pass < 2 && c->nev[pass] < 4096;
+    if (timed) cudaEventRecord(c->ev[pass][0][c->nev[pass]], c->st);
+    const int r = stream_form(c, [&](auto s) { return decltype(s)::pass(c, pass, grad); });
+    if (timed) {
+        cudaEventRecord(c->ev[pass][1][c->nev[pass]], c->st);
+        c->nev[pass]++;
+    }
+    return r;
+}
+
+/* slots -> densities, exchange, tau, potentials and coefficients at time index it (it < 0: none) */
+static int stream_after(wtd_ctx *c, bool full, int it)
+{
+    constexpr int N = WTD_NUMEL;
+    const double *s0 = c->dslot, *s1 = s0 + (size_t)c->gpt * 4 * N, *s2 = s1 + (size_t)c->gpl * 6 * N;
+    k3s_dens_reduce<<<(12 * N + 255) / 256, 256, 0, c->st>>>(s0, c->gpt, s1, c->gpl, s2, c->gx, c->dens, full ? 1 : 0, 1.0 / WTD_LPERP);
+    WTD_LAUNCHED(c);
+    WTD_TRY(exchange(c, c->dens, 12 * (size_t)N));
+    if (full) WTD_TRY(big_tau(c->dens, c->stage3d, c->tw, c->ktab, c->st));
+    if (it < 0) return WTD_OK;
+    WTD_TRY(functional(c, it));
+    return coef_with_friction(c, it);
+}
+
+static int stream_step(wtd_ctx *c, bool last)
+{
+    const bool var = WTD_VAR;
+    if (!c->fk_given && !c->have_coef) return WTD_ERR_STATE;
+    c->qfsw = 0.0;
+    WTD_TRY(stream_pass(c, 0, var));
+    WTD_TRY(stream_after(c, var, c->it + 1));
+    const bool g = var || last;
+    WTD_TRY(stream_pass(c, 1, g));
+    WTD_TRY(stream_after(c, g, c->it + 1));
+    c->head = (c->head + WTD_NHIST - 1) % WTD_NHIST;
+    c->fk_given = 0;
+    c->it++;
+    return WTD_OK;
+}
+
+/* the states in place times their scale: what every call leaves behind */
+static int stream_rescale(wtd_ctx *c)
+{
+    return stream_form(c, [&](auto s) { return decltype(s)::rescale(c); });
+}
+
+static int stream_initial(wtd_ctx *c)
+{
+    WTD_TRY(stream_pass(c, 2, true));
+    WTD_TRY(stream_after(c, true, -1));
+    return stream_rescale(c);
+}
+
+static int stream_setup(wtd_ctx *c, int nsm)
+{
+    return stream_form(c, [&](auto s) { return decltype(s)::setup(c, nsm); });
+}
+#else
+static bool stream_fits(int) { return false; }
+static size_t stream_slot_words(const wtd_ctx *) { return 0; }
+static size_t stream_part_words(const wtd_ctx *) { return 0; }
+static int stream_pass(wtd_ctx *, int, bool) { return WTD_ERR_UNSUPPORTED; }
+static int stream_step(wtd_ctx *, bool) { return WTD_ERR_UNSUPPORTED; }
+static int stream_rescale(wtd_ctx *) { return WTD_ERR_UNSUPPORTED; }
+static int stream_initial(wtd_ctx *) { return WTD_ERR_UNSUPPORTED; }
+static int stream_setup(wtd_ctx *, int) { return WTD_ERR_UNSUPPORTED; }
+#endif
 
 /* ---------------------------------------------------------------------------------------
  * line path (3D lattices beyond one CTA, wtd_path3d.cuh): per half step k3_plane_h (when H is
@@ -957,19 +1168,23 @@ int wtd_create(wtd_ctx **out, int nwf, int precision, int device)
         const char *pf = getenv("WTD_PREFETCH");
         if (pf) c->prefetch = atoi(pf) & 15;
     }
-    /* lattices beyond one CTA.  The FP32-mixed forms take the 3D line path (FP32 arithmetic,
-     * complex64 history possible); FP64 takes the staged path, which measures faster in FP64
-     * on 32^3.  WTD_3D_PATH=line or =staged selects either for every form. */
+    /* lattices beyond one CTA.  Where it fits (3D, axes of at most 64 points) every form takes the
+     * stream path; elsewhere the FP32-mixed forms take the 3D line path and FP64 the staged path,
+     * each the faster there.  WTD_3D_PATH=line selects the stream (or line) path for every form,
+     * =staged the staged path. */
     {
         const char *pp = getenv("WTD_3D_PATH");
-        bool want_line = precision != WTD_FP64;
-        if (pp && strcmp(pp, "line") == 0) want_line = true;
-        if (pp && strcmp(pp, "staged") == 0) want_line = false;
-        c->line = (WTD_BIG && line_fits(precision) && want_line) ? 1 : 0;
+        const bool stream = stream_fits(precision);
+        bool want = stream || precision != WTD_FP64;
+        if (pp && strcmp(pp, "line") == 0) want = true;
+        if (pp && strcmp(pp, "staged") == 0) want = false;
+        c->stream = (stream && want) ? 1 : 0;
+        c->line = (!c->stream && WTD_BIG && line_fits(precision) && want) ? 1 : 0;
     }
-    c->staged = (WTD_BIG && !c->line) ? 1 : 0;
+    c->staged = (WTD_BIG && !c->line && !c->stream) ? 1 : 0;
     if (c->staged && precision == WTD_MIXED_H32) { free(c); return WTD_ERR_UNSUPPORTED; }
     if (c->line && line_setup(c, nsm) != WTD_OK) { free(c); return WTD_ERR_CUDA; }
+    if (c->stream && stream_setup(c, nsm) != WTD_OK) { free(c); return WTD_ERR_CUDA; }
     int per_sm = WTD_BIG ? 2 : occupancy_per_sm(c);
     c->grid = nsm * per_sm;
     if (c->grid > nwf) c->grid = nwf;
@@ -987,6 +1202,7 @@ int wtd_create(wtd_ctx **out, int nwf, int precision, int device)
          * on the line path per cluster and per plane chunk (12 N words) */
         size_t slots = (size_t)c->grid * 16 * N;
         if (c->line && (size_t)(c->ncl + c->g2) * 12 * N > slots) slots = (size_t)(c->ncl + c->g2) * 12 * N;
+        if (c->stream && stream_slot_words(c) > slots) slots = stream_slot_words(c);
         ALLOC(c->dslot, slots * sizeof(double));
     }
     ALLOC(c->qpe, nwf * sizeof(double));
@@ -1002,9 +1218,13 @@ int wtd_create(wtd_ctx **out, int nwf, int precision, int device)
         ALLOC(c->xfer, WTD_XFER * sizeof(double2));
         if (c->staged) ALLOC(c->stage, n2 * sizeof(double2));
     }
-    if (c->line) {
+    if (c->line || c->stream) {
         ALLOC(c->kbuf, n2 * (precision == WTD_FP64 ? sizeof(double2) : sizeof(float2)));
         ALLOC(c->stage3d, 2 * N * sizeof(double2));
+    }
+    if (c->stream) {
+        ALLOC(c->sc, nwf * sizeof(double));
+        ALLOC(c->part, stream_part_words(c) * sizeof(double));
     }
     if (c->staged) {
         ALLOC(c->ddx, n2 * sizeof(double2));
@@ -1037,6 +1257,7 @@ int wtd_create(wtd_ctx **out, int nwf, int precision, int device)
         cudaMemcpy(c->kp2, h, nwf * sizeof(double), cudaMemcpyHostToDevice);
         for (int i = 0; i < nwf; i++) h[i] = 1.0;
         cudaMemcpy(c->wcnt, h, nwf * sizeof(double), cudaMemcpyHostToDevice);
+        if (c->sc) cudaMemcpy(c->sc, h, nwf * sizeof(double), cudaMemcpyHostToDevice);
         free(h);
     }
     for (int h = 0; h < WTD_NHIST; h++) cudaMemsetAsync(c->hist[h], 0, c->hsz, c->st);
@@ -1061,7 +1282,7 @@ int wtd_destroy(wtd_ctx *c)
                 for (int i = 0; i < 4096; i++) cudaEventDestroy(c->ev[p][k][i]);
     void *ptrs[] = {c->y, c->cf, c->occ, c->kp2, c->wcnt, c->dslot, c->qpe, c->dens, c->pots, c->qfld, c->dqf, c->ework,
                     c->eout, c->tw, c->ktab, c->stage, c->extra, c->ddx, c->ddy, c->ddz, c->dlap, c->dalap, c->stage3d,
-                    c->kbuf, c->xfer};
+                    c->kbuf, c->xfer, c->sc, c->part};
     for (size_t i = 0; i < sizeof(ptrs) / sizeof(ptrs[0]); i++) if (ptrs[i]) cudaFree(ptrs[i]);
     for (int h = 0; h < WTD_NHIST; h++) if (c->hist[h]) cudaFree(c->hist[h]);
     if (c->st) cudaStreamDestroy(c->st);
@@ -1261,6 +1482,10 @@ int wtd_initial_measurement(wtd_ctx *c, int it0)
         WTD_TRY(staged_initial(c));
         return wtd_cuerr(cudaGetLastError());
     }
+    if (c->stream) {
+        WTD_TRY(stream_initial(c));
+        return wtd_cuerr(cudaGetLastError());
+    }
     if (c->line) {
         WTD_TRY(line_initial(c));
         return wtd_cuerr(cudaGetLastError());
@@ -1278,6 +1503,10 @@ int wtd_steps(wtd_ctx *c, int nsteps)
     if (c->staged) {
         for (int s = 0; s < nsteps; s++) WTD_TRY(staged_step(c, s == nsteps - 1));
         return WTD_OK;
+    }
+    if (c->stream) {
+        for (int s = 0; s < nsteps; s++) WTD_TRY(stream_step(c, s == nsteps - 1));
+        return nsteps > 0 ? stream_rescale(c) : WTD_OK;
     }
     if (c->line) {
         for (int s = 0; s < nsteps; s++) WTD_TRY(line_step(c, s == nsteps - 1));
@@ -1420,19 +1649,23 @@ int wtd_set_quantum_friction(wtd_ctx *c, double alpha, double beta, double gamma
     if (!c) return WTD_ERR_ARG;
     const bool on = alpha != 0.0 || beta != 0.0 || gamma != 0.0;
     if (on && !(ramp > 0.0)) return WTD_ERR_ARG;
-    if (on && c->line) {
-        /* the line path has no friction densities: the run continues on the staged path, which
-         * keeps the same state, ring and f_k conventions (FP64 only) */
+    if (on && (c->line || c->stream)) {
+        /* these paths have no friction densities: the run continues on the staged path, which
+         * keeps the same state, ring and f_k conventions (FP64 only; the buffer of H psi becomes
+         * one of its derivative arrays) */
         if (c->prec != WTD_FP64) return WTD_ERR_UNSUPPORTED;
         WTD_CU(cudaSetDevice(c->dev));
         if (!c->fk_given && c->have_coef) WTD_TRY(ensure_fk(c));
         const size_t n2 = (size_t)2 * c->S * WTD_NUMEL;
         cudaError_t e = cudaSuccess;
         double2 **bufs[5] = {&c->ddx, &c->ddy, &c->ddz, &c->dlap, &c->dalap};
-        for (int k = 0; k < 5 && e == cudaSuccess; k++)
+        for (int k = 1; k < 5 && e == cudaSuccess; k++)
             if ((k < 4 || WTD_VAR) && !*bufs[k]) e = cudaMalloc((void **)bufs[k], n2 * sizeof(double2));
         if (e != cudaSuccess) { cudaGetLastError(); return WTD_ERR_NOMEM; }
-        c->line = 0;
+        WTD_TRY(staged_dens_chunks(c, &c->sdg));
+        c->ddx = (double2 *)c->kbuf;
+        c->kbuf = NULL;
+        c->line = c->stream = 0;
         c->staged = 1;
     }
     c->qf[0] = alpha; c->qf[1] = beta; c->qf[2] = gamma; c->qf[3] = nreq;
@@ -2060,7 +2293,7 @@ extern "C" int wtd_adjoint(wtd_ctx *c, int it0, int nsteps, int checkpoint_every
         (grad && nparam < 1))
         return WTD_ERR_ARG;
 #if defined(WTD_ADJOINT_CONTACT_BDG) && defined(FAST_CONST_EFFECTIVE_MASS_MODE) && !defined(SPINSYMMETRY_MODE)
-    if (c->prec != WTD_FP64 || c->staged || c->sstride != 12 * WTD_NUMEL) return WTD_ERR_UNSUPPORTED;
+    if (c->prec != WTD_FP64 || WTD_BIG || c->sstride != 12 * WTD_NUMEL) return WTD_ERR_UNSUPPORTED;
     WTD_CU(cudaSetDevice(c->dev));
     int r = adjoint_forward(c, it0, nsteps, checkpoint_every, mask, grad != NULL, loss);
     if (r == WTD_OK && grad) r = adjoint_reverse(c, nparam, grad);
@@ -2077,7 +2310,7 @@ extern "C" int wtd_adjoint_forward(wtd_ctx *c, int it0, int nsteps, int checkpoi
 {
     if (!c || !loss || nsteps < 1 || checkpoint_every < 0) return WTD_ERR_ARG;
 #if defined(WTD_ADJOINT_CONTACT_BDG) && defined(FAST_CONST_EFFECTIVE_MASS_MODE) && !defined(SPINSYMMETRY_MODE)
-    if (c->prec != WTD_FP64 || c->staged || c->sstride != 12 * WTD_NUMEL) return WTD_ERR_UNSUPPORTED;
+    if (c->prec != WTD_FP64 || WTD_BIG || c->sstride != 12 * WTD_NUMEL) return WTD_ERR_UNSUPPORTED;
     WTD_CU(cudaSetDevice(c->dev));
     const int r = adjoint_forward(c, it0, nsteps, checkpoint_every, mask, true, loss);
     if (r != WTD_OK) cudaStreamSynchronize(c->st);

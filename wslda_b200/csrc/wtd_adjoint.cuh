@@ -78,30 +78,52 @@ __device__ __forceinline__ void nu_adjoint(double2 &gu, double2 &gv, double2 nb,
     gv.y += cn * (nb.x * u.y - nb.y * u.x);
 }
 
+/* the reverse kernels' form on a lattice: folded circulant lines (wtd_circ.cuh) where one block of
+ * up to 256 threads holds all lines of a field, so that the laplacian is taken in place, with two
+ * CTAs per SM; else the transforms with 512 threads */
+template <class G> struct AdjCfg {
+    typedef CircGeo<G> CG;
+    static constexpr bool circ = CG::fits && CG::nmax <= 48 && CG::total <= 256;
+    typedef typename std::conditional<circ, CG, G>::type Lay;
+    static constexpr int lines = (CG::total + 31) / 32 * 32;
+    static constexpr int threads = circ ? (G::ntot >= 128 && lines < 128 ? 128 : lines)
+                                        : G::ntot >= 512 ? 512 : (G::ntot + 31) / 32 * 32;
+    static constexpr int minb = circ ? 2 : 1;
+    static constexpr size_t smem = 2 * (size_t)Lay::padded * sizeof(double2) + 80 * sizeof(double) +
+                                   (circ ? 0 : (size_t)G::twtotal * sizeof(double2) + sizeof(KTab<G>));
+};
+
 /* laplacian of the two fields in (BU, BV), in place */
 template <class G>
 __device__ __forceinline__ void lap2(double2 *BU, double2 *BV, const double2 *tw, const double (*kt)[WTD_KT])
 {
     __syncthreads();
-    fft_forward<G, 2>(BU, (int)(BV - BU), tw);
-    kmul<G, OP_LAP>(BU, kt);
-    kmul<G, OP_LAP>(BV, kt);
-    __syncthreads();
-    fft_inverse<G, 2>(BU, (int)(BV - BU), tw);
+    if constexpr (AdjCfg<G>::circ) {
+#pragma unroll 1
+        for (int comp = 0; comp < 2; comp++)
+            circ_lap<typename AdjCfg<G>::Lay, true>(comp ? BV : BU, comp ? BV : BU);
+    } else {
+        fft_forward<G, 2>(BU, (int)(BV - BU), tw);
+        kmul<G, OP_LAP>(BU, kt);
+        kmul<G, OP_LAP>(BV, kt);
+        __syncthreads();
+        fft_inverse<G, 2>(BU, (int)(BV - BU), tw);
+    }
 }
 
 /* reverse of pass B (corrector half step), persistent CTAs over states */
 template <class G, int NH>
-__global__ void __launch_bounds__(512, 1) k_adj_B(AdjArgs a, const double2 *gtw, const double *gk)
+__global__ void __launch_bounds__(AdjCfg<G>::threads, AdjCfg<G>::minb) k_adj_B(AdjArgs a, const double2 *gtw, const double *gk)
 {
     constexpr int N = G::ntot;
     extern __shared__ __align__(16) unsigned char smem_raw[];
+    typedef typename AdjCfg<G>::Lay Lay;
     double2 *BU = (double2 *)smem_raw;
-    double2 *BV = BU + G::padded;
-    double2 *tw = BV + G::padded;
+    double2 *BV = BU + Lay::padded;
+    double2 *tw = BV + Lay::padded;
     double (*kt)[WTD_KT] = (double (*)[WTD_KT])(tw + G::twtotal);
-    double *red = (double *)(kt + 6);
-    load_tables<G>(tw, kt, gtw, gk);
+    double *red = AdjCfg<G>::circ ? (double *)tw : (double *)(kt + 6);
+    if constexpr (!AdjCfg<G>::circ) load_tables<G>(tw, kt, gtw, gk);
     double *ds = a.slots + (size_t)blockIdx.x * 4 * N;
     for (int i = threadIdx.x; i < 4 * N; i += blockDim.x) ds[i] = 0.0;
     const size_t SN = (size_t)a.S * N;
@@ -115,8 +137,8 @@ __global__ void __launch_bounds__(512, 1) k_adj_B(AdjArgs a, const double2 *gtw,
         for (int p = threadIdx.x; p < N; p += blockDim.x) {
             double2 u = a.y1[bu + p], v = a.y1[bv + p], gu = a.ybar[bu + p], gv = a.ybar[bv + p];
             if (a.nubar) nu_adjoint(gu, gv, a.nubar[p], cn, u, v);
-            BU[G::off(p)] = gu;
-            BV[G::off(p)] = gv;
+            BU[Lay::off(p)] = gu;
+            BV[Lay::off(p)] = gv;
             r1 += gu.x * u.x + gu.y * u.y + gv.x * v.x + gv.y * v.y;
         }
         r1 = block_sum(r1, red);
@@ -124,7 +146,7 @@ __global__ void __launch_bounds__(512, 1) k_adj_B(AdjArgs a, const double2 *gtw,
         /* Pbar = yhbar = (ybar - dV r1 y1)/n;  fbar_p = i dt c Pbar;  s = Re<fbar_p, y_p> */
         double s = 0.0;
         for (int p = threadIdx.x; p < N; p += blockDim.x) {
-            const int o = G::off(p);
+            const int o = Lay::off(p);
             double2 u = a.y1[bu + p], v = a.y1[bv + p], gu = BU[o], gv = BV[o];
             double2 pu = make_double2((gu.x - dV * r1 * u.x) * inv_n, (gu.y - dV * r1 * u.y) * inv_n);
             double2 pv = make_double2((gv.x - dV * r1 * v.x) * inv_n, (gv.y - dV * r1 * v.y) * inv_n);
@@ -136,7 +158,7 @@ __global__ void __launch_bounds__(512, 1) k_adj_B(AdjArgs a, const double2 *gtw,
         s = block_sum(s, red);
         /* x = fbar_p - 2 s dV y_p, its laplacian in shared memory */
         for (int p = threadIdx.x; p < N; p += blockDim.x) {
-            const int o = G::off(p);
+            const int o = Lay::off(p);
             double2 pu = a.pbar[bu + p], pv = a.pbar[bv + p], yu = a.yp[bu + p], yv = a.yp[bv + p];
             BU[o] = make_double2(-dc * pu.y - 2.0 * s * dV * yu.x, dc * pu.x - 2.0 * s * dV * yu.y);
             BV[o] = make_double2(-dc * pv.y - 2.0 * s * dV * yv.x, dc * pv.x - 2.0 * s * dV * yv.y);
@@ -144,7 +166,7 @@ __global__ void __launch_bounds__(512, 1) k_adj_B(AdjArgs a, const double2 *gtw,
         lap2<G>(BU, BV, tw, kt);
         const double E = a.E[n];
         for (int p = threadIdx.x; p < N; p += blockDim.x) {
-            const int o = G::off(p);
+            const int o = Lay::off(p);
             double2 pu = a.pbar[bu + p], pv = a.pbar[bv + p], yu = a.yp[bu + p], yv = a.yp[bv + p];
             double2 fu = make_double2(-dc * pu.y, dc * pu.x), fv = make_double2(-dc * pv.y, dc * pv.x);
             double2 xu = make_double2(fu.x - 2.0 * s * dV * yu.x, fu.y - 2.0 * s * dV * yu.y);
@@ -164,17 +186,18 @@ __global__ void __launch_bounds__(512, 1) k_adj_B(AdjArgs a, const double2 *gtw,
 /* reverse of pass A (predictor half step).  has_h: f_k was formed from y_k with H of this
  * half step, so its completed adjoint (ring position 0) flows into ybar_k and the potentials */
 template <class G, int NH>
-__global__ void __launch_bounds__(512, 1) k_adj_A(AdjArgs a, const double2 *gtw, const double *gk)
+__global__ void __launch_bounds__(AdjCfg<G>::threads, AdjCfg<G>::minb) k_adj_A(AdjArgs a, const double2 *gtw, const double *gk)
 {
     typedef Abm<NH> AB;
     constexpr int N = G::ntot;
     extern __shared__ __align__(16) unsigned char smem_raw[];
+    typedef typename AdjCfg<G>::Lay Lay;
     double2 *BU = (double2 *)smem_raw;
-    double2 *BV = BU + G::padded;
-    double2 *tw = BV + G::padded;
+    double2 *BV = BU + Lay::padded;
+    double2 *tw = BV + Lay::padded;
     double (*kt)[WTD_KT] = (double (*)[WTD_KT])(tw + G::twtotal);
-    double *red = (double *)(kt + 6);
-    load_tables<G>(tw, kt, gtw, gk);
+    double *red = AdjCfg<G>::circ ? (double *)tw : (double *)(kt + 6);
+    if constexpr (!AdjCfg<G>::circ) load_tables<G>(tw, kt, gtw, gk);
     double *ds = a.slots + (size_t)blockIdx.x * 4 * N;
     if (a.has_h)
         for (int i = threadIdx.x; i < 4 * N; i += blockDim.x) ds[i] = 0.0;
@@ -189,8 +212,8 @@ __global__ void __launch_bounds__(512, 1) k_adj_A(AdjArgs a, const double2 *gtw,
         for (int p = threadIdx.x; p < N; p += blockDim.x) {
             double2 u = a.yp[bu + p], v = a.yp[bv + p], gu = a.ypbar[bu + p], gv = a.ypbar[bv + p];
             if (a.nubar) nu_adjoint(gu, gv, a.nubar[p], cn, u, v);
-            BU[G::off(p)] = gu;
-            BV[G::off(p)] = gv;
+            BU[Lay::off(p)] = gu;
+            BV[Lay::off(p)] = gv;
             r2 += gu.x * u.x + gu.y * u.y + gv.x * v.x + gv.y * v.y;
         }
         r2 = block_sum(r2, red);
@@ -199,7 +222,7 @@ __global__ void __launch_bounds__(512, 1) k_adj_A(AdjArgs a, const double2 *gtw,
          * fbar_{k-j} += i dt (b_j ytbar + a_j Pbar);  s = Re<fbar_k, y_k> */
         double s = 0.0;
         for (int p = threadIdx.x; p < N; p += blockDim.x) {
-            const int o = G::off(p);
+            const int o = Lay::off(p);
 #pragma unroll
             for (int comp = 0; comp < 2; comp++) {
                 const size_t gi = (comp ? bv : bu) + p;
@@ -224,7 +247,7 @@ __global__ void __launch_bounds__(512, 1) k_adj_A(AdjArgs a, const double2 *gtw,
         if (a.has_h) {
             s = block_sum(s, red);
             for (int p = threadIdx.x; p < N; p += blockDim.x) {
-                const int o = G::off(p);
+                const int o = Lay::off(p);
                 double2 fu = a.fring[0][bu + p], fv = a.fring[0][bv + p], yu = a.y1[bu + p], yv = a.y1[bv + p];
                 BU[o] = make_double2(fu.x - 2.0 * s * dV * yu.x, fu.y - 2.0 * s * dV * yu.y);
                 BV[o] = make_double2(fv.x - 2.0 * s * dV * yv.x, fv.y - 2.0 * s * dV * yv.y);
@@ -232,7 +255,7 @@ __global__ void __launch_bounds__(512, 1) k_adj_A(AdjArgs a, const double2 *gtw,
             lap2<G>(BU, BV, tw, kt);
             const double E = a.E[n];
             for (int p = threadIdx.x; p < N; p += blockDim.x) {
-                const int o = G::off(p);
+                const int o = Lay::off(p);
                 double2 fu = a.fring[0][bu + p], fv = a.fring[0][bv + p], yu = a.y1[bu + p], yv = a.y1[bv + p];
                 double2 xu = make_double2(fu.x - 2.0 * s * dV * yu.x, fu.y - 2.0 * s * dV * yu.y);
                 double2 xv = make_double2(fv.x - 2.0 * s * dV * yv.x, fv.y - 2.0 * s * dV * yv.y);

@@ -2173,8 +2173,7 @@ static int adjoint_reverse(wtd_ctx *c, int nparam, double *grad_h)
     constexpr int N = WTD_NUMEL, NH = WTD_NHIST;
     const int S = c->S;
     const size_t NS = (size_t)2 * S * N;
-    constexpr size_t sm = 2 * (size_t)WG::padded * sizeof(double2) + WG::twtotal * sizeof(double2) + sizeof(KTab<WG>) +
-                          80 * sizeof(double);
+    constexpr size_t sm = AdjCfg<WG>::smem;
     AdjWork *w = (AdjWork *)c->adj;
     if (!w || !w->ready || w->mark_launches != c->launches || w->mark_mut != c->mut) return WTD_ERR_STATE;
     w->ready = false;
@@ -2202,12 +2201,12 @@ static int adjoint_reverse(wtd_ctx *c, int nparam, double *grad_h)
     WTD_ONCE_PER_DEVICE(
         WTD_CU(cudaFuncSetAttribute(kB, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
         WTD_CU(cudaFuncSetAttribute(kA, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm)));
-    /* the reverse kernels: one persistent CTA of 512 threads per SM (two CTAs of 256 per SM
-     * measured the same); the slots hold c->grid * 12 N words, so up to 3 * c->grid CTAs of 4 N */
-    const int threads = WG::ntot >= 512 ? 512 : ((WG::ntot + 31) / 32) * 32;
+    /* the reverse kernels' persistent CTAs (AdjCfg); the slots hold c->grid * 12 N words, so up to
+     * 3 * c->grid CTAs of 4 N */
+    constexpr int threads = AdjCfg<WG>::threads;
     int nsm = 148;
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c->dev);
-    int agrid = nsm;
+    int agrid = nsm * AdjCfg<WG>::minb;
     if (agrid > 3 * c->grid) agrid = 3 * c->grid;
     if (agrid > S) agrid = S;
     const int nb = (N + 255) / 256;

@@ -276,20 +276,15 @@ __global__ void __launch_bounds__(AdjCfg<G>::threads, AdjCfg<G>::minb) k_adj_A(A
 #ifdef WTD_ADJOINT_CONTACT_BDG
 /* second stage of the potentials' adjoint: fixed-order sum over the per-CTA slots.
  * vbar[0..N) = Vabar, vbar[N..2N) = Vbbar; nubar = -g Deltabar */
-__global__ void k_adj_reduce(const double *slots, int nslots, double *vbar, double2 *nubar)
+__global__ void __launch_bounds__(32 * WTD_RED_W) k_adj_reduce(const double *slots, int nslots, double *vbar, double *nubar)
 {
     constexpr int N = WTD_NUMEL;
-    int p = threadIdx.x + blockIdx.x * blockDim.x;
-    if (p >= N) return;
-    double dr = 0.0, di = 0.0, va = 0.0, vb = 0.0;
-    for (int k = 0; k < nslots; k++) {
-        const double *s = slots + (size_t)k * 4 * N;
-        dr += s[2 * p]; di += s[2 * p + 1]; va += s[2 * N + p]; vb += s[3 * N + p];
-    }
-    const double g = dc_params[WTD_ADJOINT_CONTACT_BDG];
-    vbar[p] = va;
-    vbar[N + p] = vb;
-    nubar[p] = make_double2(-g * dr, -g * di);
+    __shared__ double part[WTD_RED_W][32];
+    const int i = (threadIdx.x & 31) + blockIdx.x * 32;   /* slot words: Deltabar (2 N), Vabar, Vbbar */
+    const double s = slot_sum(i < 4 * N ? nslots : 0, part, [&](int k) { return slots[(size_t)k * 4 * N + i]; });
+    if (threadIdx.x >= 32 || i >= 4 * N) return;
+    if (i < 2 * N) nubar[i] = -dc_params[WTD_ADJOINT_CONTACT_BDG] * s;
+    else vbar[i - 2 * N] = s;
 }
 
 /* part[j][chunk] = sum over this chunk of the points of (Vabar dv_ext_a/dtheta_j + Vbbar

@@ -292,7 +292,33 @@ static int filter_fields(wtd_ctx *c)
     return filter_h(c);
 }
 
-/* per-point H coefficients from the potentials at time index it (variable mass: lap alpha /4
+/* real-field kernels by folded lines on single-CTA lattices whose lines fit, else by transforms */
+static constexpr bool WTD_LINES = !WTD_BIG && CircGeo<WG>::fits;
+
+/* variable mass: lap alpha /4 and -div A /2 from the coefficients' alpha and A */
+static int coef_var(wtd_ctx *c)
+{
+    c->have_coef = 1;
+#ifndef FAST_CONST_EFFECTIVE_MASS_MODE
+    if constexpr (WTD_BIG) return big_prep_var(c->cf, c->stage3d, c->tw, c->ktab, c->st);
+    else if constexpr (WTD_LINES) {
+        constexpr size_t sm = RealLines<CircGeo<WG>>::bytes;
+        WTD_ONCE_PER_DEVICE(WTD_CU(cudaFuncSetAttribute(wtd_prep_var_lines<WG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm)));
+        wtd_prep_var_lines<WG><<<dim3(2, 2), 256, sm, c->st>>>(c->cf);
+        WTD_LAUNCHED(c);
+    } else {
+        constexpr size_t sm = (size_t)WG::padded * sizeof(double2) + WG::twtotal * sizeof(double2) + sizeof(KTab<WG>);
+        if (sm > WTD_SMEM_MAX) return WTD_ERR_UNSUPPORTED;
+        WTD_ONCE_PER_DEVICE(WTD_CU(cudaFuncSetAttribute(wtd_prep_var<WG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm)));
+        wtd_prep_var<WG><<<2, 256, sm, c->st>>>(c->cf, c->tw, c->ktab);
+        WTD_LAUNCHED(c);
+    }
+#endif
+    return WTD_OK;
+}
+
+/* per-point H coefficients from the potentials at time index it (variable
+ mass: lap alpha /4
  * and -div A /2 by spectral derivatives) */
 static int coef_from_pots(wtd_ctx *c, int it, const double *fld = NULL)
 {
@@ -305,19 +331,7 @@ static int coef_from_pots(wtd_ctx *c, int it, const double *fld = NULL)
     }
     wtd_prep_coef<<<(N + 127) / 128, 128, 0, c->st>>>(it, P, c->cf);
     WTD_LAUNCHED(c);
-#ifndef FAST_CONST_EFFECTIVE_MASS_MODE
-    if (WTD_BIG) {
-        WTD_TRY(big_prep_var(c->cf, c->stage3d, c->tw, c->ktab, c->st));
-    } else {
-        constexpr size_t sm = (size_t)WG::padded * sizeof(double2) + WG::twtotal * sizeof(double2) + sizeof(KTab<WG>);
-        if (sm > WTD_SMEM_MAX) return WTD_ERR_UNSUPPORTED;
-        WTD_ONCE_PER_DEVICE(WTD_CU(cudaFuncSetAttribute(wtd_prep_var<WG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm)));
-        wtd_prep_var<WG><<<2, 256, sm, c->st>>>(c->cf, c->tw, c->ktab);
-        WTD_LAUNCHED(c);
-    }
-#endif
-    c->have_coef = 1;
-    return WTD_OK;
+    return coef_var(c);
 }
 
 /* the functional at time index it (potentials kernel and the user's modify_potentials) */
@@ -365,26 +379,61 @@ static int coef_with_friction(wtd_ctx *c, int it)
     return WTD_OK;
 }
 
+/* tau of both spins from the laplacian of rho on a single-CTA lattice */
+static int tau_of_rho(wtd_ctx *c, double *dens)
+{
+    if constexpr (WTD_LINES) {
+        constexpr size_t sm = RealLines<CircGeo<WG>>::bytes;
+        WTD_ONCE_PER_DEVICE(WTD_CU(cudaFuncSetAttribute(wtd_tau_lines<WG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm)));
+        wtd_tau_lines<WG><<<2, 256, sm, c->st>>>(dens);
+    } else {
+        constexpr size_t sm = (size_t)WG::padded * sizeof(double2) + WG::twtotal * sizeof(double2) + sizeof(KTab<WG>);
+        if (sm > WTD_SMEM_MAX) return WTD_ERR_UNSUPPORTED;
+        WTD_ONCE_PER_DEVICE(WTD_CU(cudaFuncSetAttribute(wtd_tau_kernel<WG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm)));
+        wtd_tau_kernel<WG><<<2, 512, sm, c->st>>>(dens, c->tw, c->ktab);
+    }
+    WTD_LAUNCHED(c);
+    return WTD_OK;
+}
+
+/* the functional and the H coefficients at time index it: one launch per point where nothing comes
+ * between them */
+static int functional_coef(wtd_ctx *c, int it)
+{
+#if FUNCTIONAL != CUSTOMEDF && !defined(ENABLE_MODIFY_POTENTIALS)
+    if (c->hkf_mode < 1 && !(c->qfsw > 0.0)) {
+        constexpr int N = WTD_NUMEL;
+        wtd_pot_coef<<<(N + WTD_POT_THREADS - 1) / WTD_POT_THREADS, WTD_POT_THREADS, 0, c->st>>>(
+            it, convert_into_wslda_density(c->dens, N), convert_into_wslda_potential(c->pots, N, NULL), c->cf);
+        WTD_LAUNCHED(c);
+        return coef_var(c);
+    }
+#endif
+    WTD_TRY(functional(c, it));
+    return coef_with_friction(c, it);
+}
+
 /* densities from the slots, tau, potentials and H coefficients at time index it */
 static int after_pass(wtd_ctx *c, bool full, int it)
 {
     constexpr int N = WTD_NUMEL;
     const bool qf = c->qfsw > 0.0;
     const int words = (qf ? 16 : 12) * N;
-    wtd_dens_reduce<<<(words + 255) / 256, 256, 0, c->st>>>(c->dslot, c->grid, c->dens, N, full ? 1 : 0, 1.0 / WTD_LPERP,
+#if FUNCTIONAL != CUSTOMEDF && !defined(ENABLE_MODIFY_POTENTIALS)
+    if (!full && it >= 0 && !c->nccl && !c->xfn && c->hkf_mode < 1 && !qf) {
+        wtd_limited_after<<<(N + 31) / 32, 32 * WTD_RED_W, 0, c->st>>>(
+            c->dslot, c->grid, (size_t)c->sstride, 1.0 / WTD_LPERP, it, c->dens, convert_into_wslda_density(c->dens, N),
+            convert_into_wslda_potential(c->pots, N, NULL), c->cf);
+        WTD_LAUNCHED(c);
+        return coef_var(c);
+    }
+#endif
+    wtd_dens_reduce<<<dens_reduce_grid(words), 32 * WTD_RED_W, 0, c->st>>>(c->dslot, c->grid, c->dens, N, full ? 1 : 0, 1.0 / WTD_LPERP,
                                                             (size_t)c->sstride, words);
     WTD_LAUNCHED(c);
     WTD_TRY(exchange(c, c->dens, (size_t)words));
-    if (full) {
-        constexpr size_t sm = (size_t)WG::padded * sizeof(double2) + WG::twtotal * sizeof(double2) + sizeof(KTab<WG>);
-        if (sm > WTD_SMEM_MAX) return WTD_ERR_UNSUPPORTED;
-        WTD_ONCE_PER_DEVICE(WTD_CU(cudaFuncSetAttribute(wtd_tau_kernel<WG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm)));
-        wtd_tau_kernel<WG><<<2, 512, sm, c->st>>>(c->dens, c->tw, c->ktab);
-        WTD_LAUNCHED(c);
-    }
-    if (it < 0) return WTD_OK;
-    WTD_TRY(functional(c, it));
-    return coef_with_friction(c, it);
+    if (full) WTD_TRY(tau_of_rho(c, c->dens));
+    return it < 0 ? WTD_OK : functional_coef(c, it);
 }
 
 /* the friction switch at time t (pca_utils.c:779-790, 1055-1060): 0 when every coefficient is
@@ -455,7 +504,7 @@ static int staged_densities(wtd_ctx *c, bool grads)
     k_dens_points<<<dim3(tiles, G), WTD_DP_T, 0, c->st>>>(S, G, st_y(c), c->ddx, c->ddy, c->ddz, c->dlap, c->occ,
                                                           c->kp2, c->wcnt, c->dslot, grads ? 1 : 0);
     WTD_LAUNCHED(c);
-    wtd_dens_reduce<<<(12 * N + 255) / 256, 256, 0, c->st>>>(c->dslot, G, c->dens, N, grads ? 1 : 0, 1.0 / WTD_LPERP);
+    wtd_dens_reduce<<<dens_reduce_grid(12 * N), 32 * WTD_RED_W, 0, c->st>>>(c->dslot, G, c->dens, N, grads ? 1 : 0, 1.0 / WTD_LPERP);
     WTD_LAUNCHED(c);
     const bool qf = c->qfsw > 0.0;
     if (qf) {
@@ -486,8 +535,7 @@ static int staged_potentials(wtd_ctx *c, int it)
     wslda_potential P = convert_into_wslda_potential(c->pots, N, NULL);
     int pb = (N + 127) / 128;
     (void)D; (void)pb;
-    WTD_TRY(functional(c, it));
-    WTD_TRY(coef_with_friction(c, it));
+    WTD_TRY(functional_coef(c, it));
 #ifndef FAST_CONST_EFFECTIVE_MASS_MODE
     /* lap(alpha psi) for the variable-mass kinetic term (pca.c:1455-1456), the product with
      * alpha taken as the fields are loaded */
@@ -718,9 +766,7 @@ static int stream_after(wtd_ctx *c, bool full, int it)
     WTD_LAUNCHED(c);
     WTD_TRY(exchange(c, c->dens, 12 * (size_t)N));
     if (full) WTD_TRY(big_tau(c->dens, c->stage3d, c->tw, c->ktab, c->st));
-    if (it < 0) return WTD_OK;
-    WTD_TRY(functional(c, it));
-    return coef_with_friction(c, it);
+    return it < 0 ? WTD_OK : functional_coef(c, it);
 }
 
 static int stream_step(wtd_ctx *c, bool last)
@@ -924,14 +970,12 @@ static int line_after(wtd_ctx *c, bool full, int it)
 {
     constexpr int N = WTD_NUMEL;
     const int nslots = c->ncl + (full ? c->g2 : 0);
-    wtd_dens_reduce<<<(12 * N + 255) / 256, 256, 0, c->st>>>(c->dslot, nslots, c->dens, N, full ? 1 : 0, 1.0 / WTD_LPERP,
+    wtd_dens_reduce<<<dens_reduce_grid(12 * N), 32 * WTD_RED_W, 0, c->st>>>(c->dslot, nslots, c->dens, N, full ? 1 : 0, 1.0 / WTD_LPERP,
                                                              12 * (size_t)N, 12 * N);
     WTD_LAUNCHED(c);
     WTD_TRY(exchange(c, c->dens, 12 * (size_t)N));
     if (full) WTD_TRY(big_tau(c->dens, c->stage3d, c->tw, c->ktab, c->st));
-    if (it < 0) return WTD_OK;
-    WTD_TRY(functional(c, it));
-    return coef_with_friction(c, it);
+    return it < 0 ? WTD_OK : functional_coef(c, it);
 }
 
 static int line_step(wtd_ctx *c, bool last)
@@ -1726,7 +1770,7 @@ static int ss_densities(wtd_ctx *c, SelfWork &w, const double2 *in, int grads)
     k_dens_compat<<<c->grid, 256, 0, c->st>>>(c->S, in, w.ddx, w.ddy, w.ddz, w.dlap, c->occ, NULL, c->kp2, c->wcnt,
                                               c->dslot, grads);
     WTD_LAUNCHED(c);
-    wtd_dens_reduce<<<(12 * N + 255) / 256, 256, 0, c->st>>>(c->dslot, c->grid, c->dens, N, grads, 1.0 / WTD_LPERP);
+    wtd_dens_reduce<<<dens_reduce_grid(12 * N), 32 * WTD_RED_W, 0, c->st>>>(c->dslot, c->grid, c->dens, N, grads, 1.0 / WTD_LPERP);
     WTD_LAUNCHED(c);
     WTD_TRY(exchange(c, c->dens, 12 * (size_t)N));
     if (!grads) return WTD_OK;
@@ -1913,7 +1957,7 @@ extern "C" int wtd_subset_densities(wtd_ctx *c, const double *weights, double *h
     if (!r) {
         k_dens_compat<<<c->grid, 256, 0, c->st>>>(c->S, (const double2 *)c->y, w.ddx, w.ddy, w.ddz, w.dlap, c->occ, dw,
                                                   c->kp2, c->wcnt, c->dslot, 1);
-        wtd_dens_reduce<<<(12 * (int)N + 255) / 256, 256, 0, c->st>>>(c->dslot, c->grid, out, (int)N, 1, 1.0 / WTD_LPERP);
+        wtd_dens_reduce<<<dens_reduce_grid(12 * (int)N), 32 * WTD_RED_W, 0, c->st>>>(c->dslot, c->grid, out, (int)N, 1, 1.0 / WTD_LPERP);
         r = wtd_cuerr(cudaGetLastError());
         c->launches += 2;
     }
@@ -2237,7 +2281,7 @@ static int adjoint_reverse(wtd_ctx *c, int nparam, double *grad_h)
             b.nrm = r.nB; b.E = r.EB; b.cf = r.cfB;
             kB<<<agrid, threads, sm, c->st>>>(b, c->tw, c->ktab);
             WTD_LAUNCHED(c);
-            k_adj_reduce<<<nb, 256, 0, c->st>>>(c->dslot, agrid, vbar, nubar);
+            k_adj_reduce<<<dens_reduce_grid(4 * N), 32 * WTD_RED_W, 0, c->st>>>(c->dslot, agrid, vbar, (double *)nubar);
             WTD_LAUNCHED(c);
             WTD_TRY(exchange(c, w->fields, 4 * (size_t)N));
             WTD_TRY(theta_grad(itk[j] + 1));
@@ -2248,7 +2292,7 @@ static int adjoint_reverse(wtd_ctx *c, int nparam, double *grad_h)
             kA<<<agrid, threads, sm, c->st>>>(a, c->tw, c->ktab);
             WTD_LAUNCHED(c);
             if (r.hasH) {
-                k_adj_reduce<<<nb, 256, 0, c->st>>>(c->dslot, agrid, vbar, nubar);
+                k_adj_reduce<<<dens_reduce_grid(4 * N), 32 * WTD_RED_W, 0, c->st>>>(c->dslot, agrid, vbar, (double *)nubar);
                 WTD_LAUNCHED(c);
                 WTD_TRY(exchange(c, w->fields, 4 * (size_t)N));
                 WTD_TRY(theta_grad(itk[j]));

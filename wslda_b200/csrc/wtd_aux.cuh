@@ -8,46 +8,65 @@
 
 #include "wtd_step.cuh"
 
-/* dens[i] = sum_s slot[s][i] / L_perp over the 12N density words (fixed slot order, so the
- * result is bitwise reproducible).  Limited mode keeps nu, rho_a, rho_b and zeroes the rest,
- * as kernel_calculate_densities_limited does (pca_dens.cu:133-198). */
-__global__ void wtd_dens_reduce(const double *slots, int nslots, double *dens, int N, int full, double inv_lperp,
-                                size_t stride = 0, int words = 0)
+/* sum over the slots of one word per lane: the block's 8 warps take every 8th slot each and their
+ * partial sums are added in warp order (fixed, so the result is bitwise reproducible).  Threads of
+ * warp 0 return the total. */
+#define WTD_RED_W 8
+template <class F> __device__ __forceinline__ double slot_sum(int nslots, double (*part)[32], F word)
+{
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    double s = 0.0;
+#pragma unroll 8
+    for (int k = w; k < nslots; k += WTD_RED_W) s += word(k);
+    part[w][lane] = s;
+    __syncthreads();
+    if (w == 0) {
+#pragma unroll
+        for (int j = 1; j < WTD_RED_W; j++) s += part[j][lane];
+    }
+    return s;
+}
+
+/* dens[i] = sum_s slot[s][i] / L_perp over the 12N density words.  Limited mode keeps nu, rho_a,
+ * rho_b and zeroes the rest, as kernel_calculate_densities_limited does (pca_dens.cu:133-198).
+ * Blocks of 32 words, 8 warps: a word's 148 to 300 slots were a chain of loads of one thread (23 us
+ * at 64^2), now an eighth of that with 8 loads in flight. */
+__global__ void __launch_bounds__(32 * WTD_RED_W) wtd_dens_reduce(const double *slots, int nslots, double *dens, int N, int full,
+                                                                  double inv_lperp, size_t stride = 0, int words = 0)
 {
     /* words: 12 N, or 16 N with the quantum-friction densities [U_a, U_b, D] after them;
      * stride: slot words per CTA */
+    __shared__ double part[WTD_RED_W][32];
     if (!stride) stride = 12 * (size_t)N;
     if (!words) words = 12 * N;
-    int i = threadIdx.x + blockIdx.x * blockDim.x;
-    if (i >= words) return;
-    int q = (i < 2 * N) ? 0 : 1 + (i - 2 * N) / N; /* 0: nu, 1: rho_a, 2: tau_a, ..., 6: rho_b ... */
-    bool needed = full || q == 0 || q == 1 || q == 6 || i >= 12 * N;
-    double s = 0.0;
+    const int i = (threadIdx.x & 31) + blockIdx.x * 32;
+    const int q = (i < 2 * N) ? 0 : 1 + (i - 2 * N) / N; /* 0: nu, 1: rho_a, 2: tau_a, ..., 6: rho_b ... */
+    const bool needed = i < words && (full || q == 0 || q == 1 || q == 6 || i >= 12 * N);
+    double s;
 #ifdef SPINSYMMETRY_MODE
     /* spin-symmetric system (pca_dens.cu:55-124, 365-461; symmetrize_densities_device): both
      * spin channels take the sum of the u (f) and v (1 - f) contributions, nu and the friction
      * pairing density D count twice.  The sum is linear, so it is taken here, over the slots,
      * before the exchange between ranks. */
-    if (needed) {
-        size_t j = (size_t)i;
-        double mul = 1.0;
-        if (q == 0 || i >= 14 * N) mul = 2.0, j = (size_t)-1;
-        else if (i >= 13 * N) j = (size_t)i - N;                /* U_b <- U_a + U_b */
-        else if (i >= 12 * N) j = (size_t)i + N;                /* U_a <- U_a + U_b */
-        else if (q >= 6) j = (size_t)i - 5 * (size_t)N;          /* b <- a + b */
-        else j = (size_t)i + 5 * (size_t)N;                      /* a <- a + b */
-        if (j == (size_t)-1)
-            for (int k = 0; k < nslots; k++) s += slots[(size_t)k * stride + i];
-        else
-            for (int k = 0; k < nslots; k++) s += slots[(size_t)k * stride + i] + slots[(size_t)k * stride + j];
-        s *= mul;
-    }
+    double mul = 1.0;
+    size_t j = 0;
+    bool pair = true;
+    if (q == 0 || i >= 14 * N) mul = 2.0, pair = false;
+    else if (i >= 13 * N) j = (size_t)i - N;                /* U_b <- U_a + U_b */
+    else if (i >= 12 * N) j = (size_t)i + N;                /* U_a <- U_a + U_b */
+    else if (q >= 6) j = (size_t)i - 5 * (size_t)N;          /* b <- a + b */
+    else j = (size_t)i + 5 * (size_t)N;                      /* a <- a + b */
+    s = mul * slot_sum(needed ? nslots : 0, part, [&](int k) {
+        const double *w = slots + (size_t)k * stride;
+        return pair ? w[i] + w[j] : w[i];
+    });
 #else
-    if (needed)
-        for (int k = 0; k < nslots; k++) s += slots[(size_t)k * stride + i];
+    s = slot_sum(needed ? nslots : 0, part, [&](int k) { return slots[(size_t)k * stride + i]; });
 #endif
-    dens[i] = s * inv_lperp;
+    if (threadIdx.x < 32 && i < words) dens[i] = s * inv_lperp;
 }
+/* CTAs of wtd_dens_reduce for `words` density words */
+static inline unsigned dens_reduce_grid(int words) { return (unsigned)((words + 31) / 32); }
 
 /* the quantum-friction particle-control coefficient (N - N_req) / N_req, N = volel *
  * sum(rho_a + rho_b), N_req kept >= 1 (pca_utils.c:1063-1072; the reference reads an
@@ -114,14 +133,95 @@ __global__ void __launch_bounds__(512) wtd_tau_kernel(double *dens, const double
     }
 }
 
+/* ---------------------------------------------------------------------------------------
+ * the same operations by folded circulant lines (wtd_circ.cuh), where the lattice's lines fit:
+ * real fields, one line per thread and axis, no transforms
+ * -------------------------------------------------------------------------------------*/
+template <class CG> struct RealLines {
+    static constexpr size_t bytes = 2 * (size_t)CG::padded * sizeof(double);
+};
+/* dst (= axis 0, += others) the operator OP along axis AX of src, both padded real fields */
+template <class CG, int OP, int AX>
+__device__ __forceinline__ void real_axis(const double *src, double *dst)
+{
+    constexpr int n = CG::n(AX), lines = CG::ntot / n;
+    for (int l = threadIdx.x; l < lines; l += blockDim.x) {
+        int e, st;   /* first element and step */
+        if (CG::dims == 1) { e = 0; st = 1; }
+        else if (AX == CG::dims - 1) { e = l * CG::pitch; st = 1; }
+        else if (AX == 0) {
+            e = CG::dims == 2 ? l : (l / CG::n(2)) * CG::pitch + l % CG::n(2);
+            st = CG::dims == 2 ? CG::pitch : CG::n(1) * CG::pitch;
+        } else { e = (l / CG::n(2)) * CG::n(1) * CG::pitch + l % CG::n(2); st = CG::pitch; }
+        double v[n];
+        circ::MemLine<double> f{src + e, st};
+        circ::line_from<OP, AX, n>(f, v);
+#pragma unroll
+        for (int j = 0; j < n; j++) dst[e + j * st] = AX > 0 ? dst[e + j * st] + v[j] : v[j];
+    }
+    __syncthreads();
+}
+template <class CG> __device__ __forceinline__ void real_load(double *B, const double *f)
+{
+    for (int p = threadIdx.x; p < CG::ntot; p += blockDim.x) B[CG::off(p)] = f[p];
+    __syncthreads();
+}
+template <class CG> __device__ __forceinline__ void real_lap(const double *src, double *dst)
+{
+    real_axis<CG, circ::LAP, 0>(src, dst);
+    if constexpr (CG::dims > 1) real_axis<CG, circ::LAP, 1>(src, dst);
+    if constexpr (CG::dims > 2) real_axis<CG, circ::LAP, 2>(src, dst);
+}
+
+/* tau_s = max(0, lap(rho_s)/2 - tau_s); blockIdx.x = spin.  12^3: two transforms of the field were
+ * two thirds of this launch's time */
+template <class G>
+__global__ void __launch_bounds__(256) wtd_tau_lines(double *dens)
+{
+    typedef CircGeo<G> CG;
+    constexpr int N = G::ntot;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    double *S = (double *)smem_raw, *D = S + CG::padded;
+    const double *rho = dens + (blockIdx.x == 0 ? 2 : 7) * (size_t)N;
+    double *tau = dens + (blockIdx.x == 0 ? 3 : 8) * (size_t)N;
+    real_load<CG>(S, rho);
+    real_lap<CG>(S, D);
+    for (int p = threadIdx.x; p < N; p += blockDim.x) {
+        const double t = 0.5 * D[CG::off(p)] - tau[p];
+        tau[p] = t < 0.0 ? 0.0 : t;
+    }
+}
+
+/* lap(alpha_s)/4 (blockIdx.y = 0) and -div(A_s)/2 (1) of the H coefficients; blockIdx.x = spin */
+template <class G>
+__global__ void __launch_bounds__(256) wtd_prep_var_lines(double *cf)
+{
+    typedef CircGeo<G> CG;
+    constexpr int N = G::ntot;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    double *S = (double *)smem_raw, *D = S + CG::padded;
+    const int s = blockIdx.x;
+    if (blockIdx.y == 0) {
+        real_load<CG>(S, cf + (s == 0 ? CF_ALA : CF_ALB) * (size_t)N);
+        real_lap<CG>(S, D);
+    } else {
+        const double *A = cf + (s == 0 ? CF_AAX : CF_ABX) * (size_t)N;
+        real_load<CG>(S, A);
+        real_axis<CG, circ::DER, 0>(S, D);
+        if constexpr (CG::dims > 1) { real_load<CG>(S, A + N); real_axis<CG, circ::DER, 1>(S, D); }
+        if constexpr (CG::dims > 2) { real_load<CG>(S, A + 2 * (size_t)N); real_axis<CG, circ::DER, 2>(S, D); }
+    }
+    double *out = cf + (blockIdx.y == 0 ? (s == 0 ? CF_NA : CF_NB) : (s == 0 ? CF_CJA : CF_CJB)) * (size_t)N;
+    const double f = blockIdx.y == 0 ? 0.25 : -0.5;
+    for (int p = threadIdx.x; p < N; p += blockDim.x) out[p] = f * D[CG::off(p)];
+}
+
 /* per-point coefficients of H psi (see the CF_* list) from the potentials at time index it.
  * Delta includes Delta_ext (pca_kernels.cu:271-276); constant mass uses -alpha/2, variable
  * mass -alpha/4 (pca_kernels.cu:296-309); BdG uses -1/2 (pca_kernels.cu:478-482). */
-__global__ void wtd_prep_coef(int it, wslda_potential P, double *cf)
+__device__ __forceinline__ void wtd_coef_point(int i, int it, const wslda_potential &P, double *cf)
 {
-    int i = threadIdx.x + blockIdx.x * blockDim.x;
     constexpr int N = WTD_NUMEL;
-    if (i >= N) return;
     int ix, iy, iz; wtd_decode(i, ix, iy, iz);
     Complex D = P.delta[i];
 #ifdef ENABLE_DELTA_EXT
@@ -167,6 +267,78 @@ __global__ void wtd_prep_coef(int it, wslda_potential P, double *cf)
     cf[CF_ABZ * N + i] = Ab[2];
 #endif
 }
+__global__ void wtd_prep_coef(int it, wslda_potential P, double *cf)
+{
+    const int i = threadIdx.x + blockIdx.x * blockDim.x;
+    if (i < WTD_NUMEL) wtd_coef_point(i, it, P, cf);
+}
+
+#if FUNCTIONAL != CUSTOMEDF && !defined(ENABLE_MODIFY_POTENTIALS)
+/* the functional and the H coefficients of each point in one launch, where nothing (a filter, the
+ * friction terms, the user's modify_potentials) comes between them */
+__global__ void __launch_bounds__(WTD_POT_THREADS) wtd_pot_coef(int it, wslda_density D, wslda_potential P, double *cf)
+{
+    const int i = threadIdx.x + blockIdx.x * blockDim.x;
+    if (i >= WTD_NUMEL) return;
+    wtd_potentials_point(i, it, D, P, 1.0);
+    wtd_coef_point(i, it, P, cf);
+}
+
+/* a half step without gradients, for a context that is the whole system: the slot sums of nu,
+ * rho_a, rho_b (wtd_dens_reduce, limited), the functional and the H coefficients of 32 points per
+ * block in one launch.  The sums and their order are those of wtd_dens_reduce. */
+__global__ void __launch_bounds__(32 * WTD_RED_W) wtd_limited_after(const double *slots, int nslots, size_t stride, double inv_lperp,
+                                                                    int it, double *dens, wslda_density D, wslda_potential P,
+                                                                    double *cf)
+{
+    constexpr size_t N = WTD_NUMEL;
+    __shared__ double part[4][WTD_RED_W][32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, i = lane + blockIdx.x * 32;
+    const bool on = i < (int)N;
+    double s[4] = {0.0, 0.0, 0.0, 0.0};
+    if (on) {
+#pragma unroll 4
+        for (int k = w; k < nslots; k += WTD_RED_W) {
+            const double *q = slots + (size_t)k * stride;
+            s[0] += q[2 * i];
+            s[1] += q[2 * i + 1];
+#ifdef SPINSYMMETRY_MODE
+            const double t = q[2 * N + i] + q[7 * N + i];
+            s[2] += t;
+            s[3] += q[7 * N + i] + q[2 * N + i];
+#else
+            s[2] += q[2 * N + i];
+            s[3] += q[7 * N + i];
+#endif
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < 4; j++) part[j][w][lane] = s[j];
+    __syncthreads();
+    if (!on) return;
+    if (w > 0) {
+        /* the eight words of tau and j are zero in this half step */
+        const int z = w - 1;                                   /* 0..6 of tau_a, j_a, tau_b, j_b */
+        dens[(size_t)(z < 4 ? 3 + z : 4 + z) * N + i] = 0.0;
+        if (w == 1) dens[11 * N + i] = 0.0;
+        return;
+    }
+#pragma unroll
+    for (int k = 1; k < WTD_RED_W; k++)
+#pragma unroll
+        for (int j = 0; j < 4; j++) s[j] += part[j][k][lane];
+#ifdef SPINSYMMETRY_MODE
+    s[0] *= 2.0;
+    s[1] *= 2.0;
+#endif
+    dens[2 * i] = s[0] * inv_lperp;
+    dens[2 * i + 1] = s[1] * inv_lperp;
+    dens[2 * N + i] = s[2] * inv_lperp;
+    dens[7 * N + i] = s[3] * inv_lperp;
+    wtd_potentials_point(i, it, D, P, 1.0);
+    wtd_coef_point(i, it, P, cf);
+}
+#endif
 
 /* variable mass: lap(alpha_s)/4 and -div(A_s)/2 by spectral derivatives of real fields
  * (pca_kernels.cu:778-795; pca_derivative.cu:490-700).  blockIdx.x = spin. */

@@ -651,7 +651,7 @@ static int calculate_densities_noalloc_impl(int n, wtd_z *wf, wtd_z *dx, wtd_z *
     if ((size_t)G > cap / per_cta) G = (int)(cap / per_cta);
     k_dens_noalloc<<<G, 256>>>(n, (const double2 *)wf, (const double2 *)dx, (const double2 *)dy, (const double2 *)dz,
                                (const double2 *)lap, fb, w, kky, kkz, cnt, slots, grads);
-    wtd_dens_reduce<<<(12 * WTD_NUMEL + 255) / 256, 256>>>(slots, G, dens, WTD_NUMEL, grads ? 1 : 0, 1.0 / WTD_LPERP);
+    wtd_dens_reduce<<<dens_reduce_grid(12 * WTD_NUMEL), 32 * WTD_RED_W>>>(slots, G, dens, WTD_NUMEL, grads ? 1 : 0, 1.0 / WTD_LPERP);
     return cu_sync_status();
 }
 
@@ -901,7 +901,7 @@ static int calculate_densities_impl(int n, wtd_z *wf, wtd_z *dx, wtd_z *dy, wtd_
     int G = g_dens_grid < n ? g_dens_grid : n;
     k_dens_compat<<<G, 256>>>(n, (const double2 *)wf, (const double2 *)dx, (const double2 *)dy, (const double2 *)dz,
                               (const double2 *)lap, fb, w, g_kp2, g_wcnt, slots, grads);
-    wtd_dens_reduce<<<(12 * WTD_NUMEL + 255) / 256, 256>>>(slots, G, dens, WTD_NUMEL, grads ? 1 : 0, 1.0 / WTD_LPERP);
+    wtd_dens_reduce<<<dens_reduce_grid(12 * WTD_NUMEL), 32 * WTD_RED_W>>>(slots, G, dens, WTD_NUMEL, grads ? 1 : 0, 1.0 / WTD_LPERP);
     return cu_sync_status();
 }
 

@@ -141,6 +141,25 @@ def test_c5_slda3d_small_s(has_gpu, monkeypatch, path):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("nwf", [2, 7, 130])
+def test_t3d_ragged_stream_path(has_gpu, nwf):
+    """3D beyond one CTA with unequal axes (20 x 18 x 22: circulant lines with odd factors, 4 columns
+    per block of the x kernels, a partial last group of states) in FP64"""
+    _compare("t3d_ragged", nwf=nwf, nsteps=3, nmeas=2)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("nwf,prec", [(7, 1), (9, 2)])
+def test_t3d_ragged_mixed_forms(has_gpu, nwf, prec):
+    """the same lattice in the FP32-mixed forms, to FP32 rounding over a block as
+    test_mixed_forms_track_fp64"""
+    o, g = run_oracle("t3d_ragged", nwf, 3, 1), run_gpu("t3d_ragged", nwf, 3, 1, precision=prec)
+    errs = density_errors(g["densities"], o["densities"], o["densities"].size // 12)
+    for k in ("rho_a", "rho_b", "nu"):
+        assert errs[k] < 1e-5, (prec, k, errs[k])
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("name,nwf,nsteps,mode", [("t1d_aslda", 24, 3, 1), ("t3d_aslda", 24, 3, 1), ("c3_aslda3d", 8, 2, 1),
                                                   ("t2d_slda", 24, 3, 2), ("t3d_aslda", 24, 3, 2), ("c3_aslda3d", 8, 2, 2),
                                                   ("t2d_vext", 24, 3, 2)])

@@ -226,6 +226,7 @@ static int run_pass(wtd_ctx *c, int pass, bool grad)
 
 static int line_pass(wtd_ctx *c, int pass, bool grad, const StepArgs *given = NULL);
 static int stream_pass(wtd_ctx *c, int pass, bool grad);
+static int stream_coef_var(wtd_ctx *c);
 
 /* f1 = (H - <H>) psi of the current state and its quasiparticle energies, as the reference
  * leaves them after a step (pca.c:1565, d_workarea[0..n)); later steps reuse f1 */
@@ -300,6 +301,7 @@ static int coef_var(wtd_ctx *c)
 {
     c->have_coef = 1;
 #ifndef FAST_CONST_EFFECTIVE_MASS_MODE
+    if (c->stream) return stream_coef_var(c);
     if constexpr (WTD_BIG) return big_prep_var(c->cf, c->stage3d, c->tw, c->ktab, c->st);
     else if constexpr (WTD_LINES) {
         constexpr size_t sm = RealLines<CircGeo<WG>>::bytes;
@@ -674,13 +676,19 @@ template <typename TY, typename TH, typename TC> struct Stream {
         }
         WTD_TRY(p == 0 ? abm<0>(c, a) : p == 1 ? abm<1>(c, a) : p == 2 ? abm<2>(c, a) : abm<3>(c, a));
         if (p == 3) return WTD_OK;
+        return dens(c, c->wcnt, grad);
+    }
+    /* density sums of the current states with per-state weights w */
+    static int dens(wtd_ctx *c, const double *w, bool grad)
+    {
         constexpr int N = S3::N;
-        k3s_dens_points<TY><<<dim3((N + 127) / 128, c->gpt), 128, 0, c->st>>>(c->S, c->gpt, y, c->sc, c->occ, c->wcnt, slots(c, 0));
+        const TY *y = (const TY *)c->y;
+        k3s_dens_points<TY><<<dim3((N + 127) / 128, c->gpt), 128, 0, c->st>>>(c->S, c->gpt, y, c->sc, c->occ, w, slots(c, 0));
         WTD_LAUNCHED(c);
         if (grad) {
-            k3s_dens_plane<TY, TC><<<2 * NX * c->gpl, S3::LT, DS::pbytes, c->st>>>(c->S, c->gpl, y, c->sc, c->occ, c->wcnt, slots(c, 1));
+            k3s_dens_plane<TY, TC><<<2 * NX * c->gpl, S3::LT, DS::pbytes, c->st>>>(c->S, c->gpl, y, c->sc, c->occ, w, slots(c, 1));
             WTD_LAUNCHED(c);
-            k3s_dens_x<TY, TC><<<S3::NQB * c->gx, 2 * S3::XL, DS::xbytes, c->st>>>(c->S, c->gx, y, c->sc, c->occ, c->wcnt, slots(c, 2));
+            k3s_dens_x<TY, TC><<<S3::NQB * c->gx, 2 * S3::XL, DS::xbytes, c->st>>>(c->S, c->gx, y, c->sc, c->occ, w, slots(c, 2));
             WTD_LAUNCHED(c);
         }
         return WTD_OK;
@@ -699,9 +707,9 @@ template <typename TY, typename TH, typename TC> struct Stream {
     static int chunks(int nsm, int occ, int unit, int S, int per)
     {
         const int slots = nsm * (occ > 0 ? occ : 1), it = (S + per - 1) / per;
-        int n = (4 * slots + unit - 1) / unit;
+        int n = 4 * slots / unit;            /* rounded down: a few CTAs more are one more round */
         if (n > it / 8) n = it / 8;
-        const int one = (slots + unit - 1) / unit;
+        const int one = slots / unit;
         if (n < one) n = one;
         return n > it ? it : n < 1 ? 1 : n;
     }
@@ -715,7 +723,7 @@ template <typename TY, typename TH, typename TC> struct Stream {
         c->xgrid = S3::NQB * chunks(nsm, o, S3::NQB, c->S, XS::NS);
         /* density slots are memory and a later sum: one round of resident CTAs */
         auto one = [&](int occ, int unit) {
-            const int n = (nsm * (occ > 0 ? occ : 1) + unit - 1) / unit;
+            const int n = nsm * (occ > 0 ? occ : 1) / unit;
             return n < 1 ? 1 : n > c->S ? c->S : n;
         };
         WTD_CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, k3s_dens_points<TY>, 128, 0));
@@ -728,6 +736,33 @@ template <typename TY, typename TH, typename TC> struct Stream {
     }
 };
 } // namespace
+
+/* lap alpha /4 and -div A /2 of the coefficients, and tau of both spins, axis by axis */
+static int stream_coef_var(wtd_ctx *c)
+{
+    if constexpr (S3::ok) {
+        k3s_coef_axis<0><<<dim3((S3Line<0>::lines + 63) / 64, 4), 64, 0, c->st>>>(c->cf);
+        WTD_LAUNCHED(c);
+        k3s_coef_axis<1><<<dim3((S3Line<1>::lines + 63) / 64, 4), 64, 0, c->st>>>(c->cf);
+        WTD_LAUNCHED(c);
+        k3s_coef_axis<2><<<dim3((S3Line<2>::lines + 63) / 64, 4), 64, 0, c->st>>>(c->cf);
+        WTD_LAUNCHED(c);
+        return WTD_OK;
+    } else return WTD_ERR_UNSUPPORTED;
+}
+static int stream_tau(wtd_ctx *c, double *dens)
+{
+    if constexpr (S3::ok) {
+        double *tmp = (double *)c->stage3d;
+        k3s_tau_axis<0><<<dim3((S3Line<0>::lines + 63) / 64, 2), 64, 0, c->st>>>(dens, tmp);
+        WTD_LAUNCHED(c);
+        k3s_tau_axis<1><<<dim3((S3Line<1>::lines + 63) / 64, 2), 64, 0, c->st>>>(dens, tmp);
+        WTD_LAUNCHED(c);
+        k3s_tau_axis<2><<<dim3((S3Line<2>::lines + 63) / 64, 2), 64, 0, c->st>>>(dens, tmp);
+        WTD_LAUNCHED(c);
+        return WTD_OK;
+    } else return WTD_ERR_UNSUPPORTED;
+}
 
 /* f(Stream of the context's precision form) */
 template <class F> static int stream_form(wtd_ctx *c, F f)
@@ -757,15 +792,32 @@ static int stream_pass(wtd_ctx *c, int pass, bool grad)
     return r;
 }
 
+static int stream_reduce(wtd_ctx *c, double *dens, bool full)
+{
+    constexpr int N = WTD_NUMEL;
+    const double *s0 = c->dslot, *s1 = s0 + (size_t)c->gpt * 4 * N, *s2 = s1 + (size_t)c->gpl * 6 * N;
+    k3s_dens_reduce<<<(12 * N + 255) / 256, 256, 0, c->st>>>(s0, c->gpt, s1, c->gpl, s2, c->gx, dens, full ? 1 : 0, 1.0 / WTD_LPERP);
+    WTD_LAUNCHED(c);
+    return WTD_OK;
+}
+
+/* densities (tau from the sum over ranks) of the current states with per-state weights w (3D states
+ * have no degeneracy weights of their own) */
+static int stream_subset(wtd_ctx *c, const double *w, double *dens)
+{
+    WTD_TRY(stream_form(c, [&](auto s) { return decltype(s)::dens(c, w, true); }));
+    WTD_TRY(stream_reduce(c, dens, true));
+    WTD_TRY(exchange(c, dens, 12 * (size_t)WTD_NUMEL));
+    return stream_tau(c, dens);
+}
+
 /* slots -> densities, exchange, tau, potentials and coefficients at time index it (it < 0: none) */
 static int stream_after(wtd_ctx *c, bool full, int it)
 {
     constexpr int N = WTD_NUMEL;
-    const double *s0 = c->dslot, *s1 = s0 + (size_t)c->gpt * 4 * N, *s2 = s1 + (size_t)c->gpl * 6 * N;
-    k3s_dens_reduce<<<(12 * N + 255) / 256, 256, 0, c->st>>>(s0, c->gpt, s1, c->gpl, s2, c->gx, c->dens, full ? 1 : 0, 1.0 / WTD_LPERP);
-    WTD_LAUNCHED(c);
+    WTD_TRY(stream_reduce(c, c->dens, full));
     WTD_TRY(exchange(c, c->dens, 12 * (size_t)N));
-    if (full) WTD_TRY(big_tau(c->dens, c->stage3d, c->tw, c->ktab, c->st));
+    if (full) WTD_TRY(stream_tau(c, c->dens));
     return it < 0 ? WTD_OK : functional_coef(c, it);
 }
 
@@ -804,6 +856,7 @@ static int stream_setup(wtd_ctx *c, int nsm)
 }
 #else
 static bool stream_fits(int) { return false; }
+static int stream_coef_var(wtd_ctx *) { return WTD_ERR_UNSUPPORTED; }
 static size_t stream_slot_words(const wtd_ctx *) { return 0; }
 static size_t stream_part_words(const wtd_ctx *) { return 0; }
 static int stream_pass(wtd_ctx *, int, bool) { return WTD_ERR_UNSUPPORTED; }
@@ -811,6 +864,7 @@ static int stream_step(wtd_ctx *, bool) { return WTD_ERR_UNSUPPORTED; }
 static int stream_rescale(wtd_ctx *) { return WTD_ERR_UNSUPPORTED; }
 static int stream_initial(wtd_ctx *) { return WTD_ERR_UNSUPPORTED; }
 static int stream_setup(wtd_ctx *, int) { return WTD_ERR_UNSUPPORTED; }
+static int stream_subset(wtd_ctx *, const double *, double *) { return WTD_ERR_UNSUPPORTED; }
 #endif
 
 /* ---------------------------------------------------------------------------------------
@@ -1909,7 +1963,9 @@ extern "C" int wtd_selfstart(wtd_ctx *c)
     if (c->staged) {
         w.ddx = c->ddx; w.ddy = c->ddy; w.ddz = c->ddz; w.dlap = c->dlap; w.dalap = c->dalap;
     } else {
-        r = get(&w.ddx, NS);
+        /* the stream and line paths' buffer of H psi is free between calls */
+        if (c->kbuf) w.ddx = (double2 *)c->kbuf;
+        else r = get(&w.ddx, NS);
         if (!r && CODEDIM >= 2) r = get(&w.ddy, NS);
         if (!r && CODEDIM >= 3) r = get(&w.ddz, NS);
         if (!r) r = get(&w.dlap, NS);
@@ -1944,7 +2000,7 @@ extern "C" int wtd_subset_densities(wtd_ctx *c, const double *weights, double *h
     int r = WTD_OK;
     if (c->staged) {
         w.ddx = c->ddx; w.ddy = c->ddy; w.ddz = c->ddz; w.dlap = c->dlap;
-    } else {
+    } else if (!c->stream) {
         r = get((void **)&w.ddx, NS * sizeof(double2));
         if (!r && CODEDIM >= 2) r = get((void **)&w.ddy, NS * sizeof(double2));
         if (!r && CODEDIM >= 3) r = get((void **)&w.ddz, NS * sizeof(double2));
@@ -1953,6 +2009,13 @@ extern "C" int wtd_subset_densities(wtd_ctx *c, const double *weights, double *h
     if (!r) r = get((void **)&dw, c->S * sizeof(double));
     if (!r) r = get((void **)&out, 12 * N * sizeof(double));
     if (!r) r = wtd_cuerr(cudaMemcpyAsync(dw, weights, c->S * sizeof(double), cudaMemcpyHostToDevice, c->st));
+    if (!r && c->stream) {
+        r = stream_subset(c, dw, out);
+        if (!r) r = wtd_cuerr(cudaMemcpyAsync(host12, out, 12 * N * sizeof(double), cudaMemcpyDeviceToHost, c->st));
+        cudaStreamSynchronize(c->st);
+        for (void *q : w.own) cudaFree(q);
+        return r;
+    }
     if (!r) r = ss_derivs(c, w, (const double2 *)c->y, 1);
     if (!r) {
         k_dens_compat<<<c->grid, 256, 0, c->st>>>(c->S, (const double2 *)c->y, w.ddx, w.ddy, w.ddz, w.dlap, c->occ, dw,

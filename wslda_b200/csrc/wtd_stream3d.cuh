@@ -90,6 +90,8 @@ k3s_plane_h(const TY *__restrict__ Y, typename cplx<TC>::t *__restrict__ K, cons
         const int n = n0 + slot;
         const bool act = n < S;
         const size_t base = ((size_t)comp * S + n) * N + (size_t)x * NYZ;
+        /* the plane of the CTA's next state on its way to L2 while this one is worked on */
+        if (t == 0 && n + NS * nch < S) prefetch_l2(Y + base + (size_t)NS * nch * N, NYZ * sizeof(TY));
         __syncthreads();
         if (act) {
             const TC s = (TC)sc[n];
@@ -193,6 +195,13 @@ template <typename TC, bool VAR> struct S3XSmem {
     static constexpr size_t bytes = slabs + NS * state;
 };
 
+/* barrier of the T threads that work on one state (whole warps where T is, else within the warp) */
+template <int T> __device__ __forceinline__ void state_sync(int slot)
+{
+    if constexpr (T >= 64) asm volatile("bar.sync %0, %1;" ::"r"(1 + slot), "n"(T) : "memory");
+    else __syncwarp();
+}
+
 template <typename TY, typename TC, bool VAR>
 __global__ void __launch_bounds__(2 * S3::XL * S3XSmem<TC, VAR>::NS)
 k3s_x_h(const TY *__restrict__ Y, typename cplx<TC>::t *K, const double *__restrict__ cf, const double *__restrict__ sc,
@@ -242,6 +251,15 @@ k3s_x_h(const TY *__restrict__ Y, typename cplx<TC>::t *K, const double *__restr
         const bool act = n < S;
         const size_t base = ((size_t)comp * S + n) * N + q0 + q;     /* complex element (x = 0) */
         TC f[NX], l[NX];
+        /* row segments of the CTA's next state (psi and K) on their way to L2 */
+        if (n + NS * nch < S) {
+            const size_t nb = ((size_t)comp * S + n + NS * nch) * N + q0;
+            for (int r = lane; r < 2 * NX; r += XL) {
+                const size_t o = nb + (size_t)(r >> 1) * NYZ;
+                if (r & 1) prefetch_l2(K + o, QB * sizeof(C));
+                else prefetch_l2(Y + o, QB * sizeof(TY));
+            }
+        }
         if (act) {
             const TC *yr = (const TC *)Y + 2 * base + c;
             const TC s = (TC)sc[n];
@@ -258,7 +276,7 @@ k3s_x_h(const TY *__restrict__ Y, typename cplx<TC>::t *K, const double *__restr
                 for (int x = 0; x < NX; x++) Hr[2 * (x * QB + q) + 1 - c] = sd * Ax[x * QB + q] * l[x];
             }
         }
-        __syncthreads();
+        state_sync<2 * XL>(slot);
         double e = 0.0;
         if (act) {
             circ::line_op<circ::LAP, 0, NX>(f, l);
@@ -291,7 +309,7 @@ k3s_x_h(const TY *__restrict__ Y, typename cplx<TC>::t *K, const double *__restr
 #pragma unroll
         for (int o = XL / 2; o > 0; o >>= 1) e += __shfl_xor_sync(0xffffffffu, e, o, XL < 32 ? XL : 32);
         if (act && lane == 0) epart[(size_t)n * (2 * S3::NQB) + 2 * qb + comp] = e;
-        __syncthreads();
+        state_sync<2 * XL>(slot);
     }
 }
 
@@ -488,6 +506,7 @@ __global__ void __launch_bounds__(S3::LT) k3s_dens_plane(int S, int nchunk, cons
         const size_t base = ((size_t)comp * S + n) * N + (size_t)x * NYZ;
         const double f0 = occ[n], w = (comp ? 1.0 - f0 : f0) * wcnt[n], wj = w * jsgn;
         const TC s = (TC)sc[n];
+        if (t == 0 && n + 1 < s1) prefetch_l2(Y + base + N, NYZ * sizeof(TY));
         __syncthreads();
 #pragma unroll 8
         for (int i = t; i < NYZ; i += LT) {
@@ -566,6 +585,8 @@ __global__ void __launch_bounds__(2 * S3::XL) k3s_dens_x(int S, int nchunk, cons
         const TC *yr = (const TC *)Y + 2 * (((size_t)comp * S + n) * N + q0 + q) + c;
         const double f0 = occ[n], w = (comp ? 1.0 - f0 : f0) * wcnt[n], wj = w * jsgn;
         const TC s = (TC)sc[n];
+        if (n + 1 < s1)
+            for (int r = lane; r < NX; r += XL) prefetch_l2(Y + ((size_t)comp * S + n + 1) * N + (size_t)r * NYZ + q0, QB * sizeof(TY));
         TC f[NX], l[NX];
 #pragma unroll
         for (int x = 0; x < NX; x++) f[x] = yr[(size_t)2 * x * NYZ];
@@ -621,6 +642,60 @@ __global__ void __launch_bounds__(256) k3s_dens_reduce(const double *sp, int gp,
     else s += total(i < 7 * N ? i + 5 * N : i - 5 * N);
 #endif
     dens[i] = s * inv_lperp;
+}
+
+/* ---------------------------------------------------------------------------------------
+ * derivatives of the O(N) real fields, one thread per line, one launch per axis for all fields
+ * (the transforms of wtd_fft3d.cuh took 40 launches for the coefficients and 10 for tau, which is
+ * most of a half step of few states)
+ * -------------------------------------------------------------------------------------*/
+template <int AX> struct S3Line {
+    static constexpr int n = AX == 0 ? NX : AX == 1 ? NY : NZ, lines = S3::N / n;
+    int base;
+    static constexpr int st = AX == 0 ? S3::NYZ : AX == 1 ? NZ : 1;
+    __device__ __forceinline__ S3Line(int l) { base = AX == 0 ? l : AX == 1 ? (l / NZ) * S3::NYZ + l % NZ : l * NZ; }
+};
+/* lap(alpha_s)/4 (blockIdx.y = 0, 1) and -div(A_s)/2 (2, 3): axis AX's part, added to the earlier */
+template <int AX>
+__global__ void __launch_bounds__(64) k3s_coef_axis(double *cf)
+{
+    typedef S3Line<AX> L;
+    const int l = threadIdx.x + blockIdx.x * 64, o = blockIdx.y, s = o & 1;
+    if (l >= L::lines) return;
+    const L line(l);
+    const double *src = cf + (size_t)(o < 2 ? CF_ALA + s : (s ? CF_ABX : CF_AAX) + AX) * S3::N + line.base;
+    double *dst = cf + (size_t)(o < 2 ? CF_NA + s : CF_CJA + s) * S3::N + line.base;
+    double v[L::n];
+    circ::MemLine<double> f{src, L::st};
+    if (o < 2) circ::line_from<circ::LAP, AX, L::n>(f, v);
+    else circ::line_from<circ::DER, AX, L::n>(f, v);
+    const double w = o < 2 ? 0.25 : -0.5;
+#pragma unroll
+    for (int j = 0; j < L::n; j++) dst[j * L::st] = AX > 0 ? dst[j * L::st] + w * v[j] : w * v[j];
+}
+/* tau_s = max(0, lap(rho_s)/2 - tau_s) (pca_dens.cu:275-338), the laplacian gathered in tmp over the
+ * axes; blockIdx.y = spin */
+template <int AX>
+__global__ void __launch_bounds__(64) k3s_tau_axis(double *dens, double *tmp)
+{
+    typedef S3Line<AX> L;
+    const int l = threadIdx.x + blockIdx.x * 64, s = blockIdx.y;
+    if (l >= L::lines) return;
+    const L line(l);
+    double v[L::n], *t = tmp + (size_t)s * S3::N + line.base;
+    circ::MemLine<double> f{dens + (size_t)(s ? 7 : 2) * S3::N + line.base, L::st};
+    circ::line_from<circ::LAP, AX, L::n>(f, v);
+    if (AX < 2) {
+#pragma unroll
+        for (int j = 0; j < L::n; j++) t[j * L::st] = AX > 0 ? t[j * L::st] + v[j] : v[j];
+    } else {
+        double *tau = dens + (size_t)(s ? 8 : 3) * S3::N + line.base;
+#pragma unroll
+        for (int j = 0; j < L::n; j++) {
+            const double r = 0.5 * (t[j * L::st] + v[j]) - tau[j * L::st];
+            tau[j * L::st] = r < 0.0 ? 0.0 : r;
+        }
+    }
 }
 
 #endif /* CODEDIM == 3 */

@@ -282,6 +282,63 @@ __global__ void __launch_bounds__(WTD_SEP_NT) k_sep_pencils(const double2 *__res
     }
 }
 
+#if CODEDIM == 2
+/* k_sep_planes in 2D, where a plane is one row: several rows per CTA (a row of 96 points is 12
+ * radix-8 butterflies, so a CTA for each left most of its threads idle: 270 us for 148 MB of
+ * states) */
+#define WTD_ROWS_CAP (2048 / (NY) >= 16 ? 16 : 2048 / (NY) >= 8 ? 8 : 2048 / (NY) >= 4 ? 4 : 2048 / (NY) >= 2 ? 2 : 1)
+typedef Geo<WTD_ROWS_CAP, NY, 1> WGR;
+static constexpr size_t sep_rows_smem = 2 * (size_t)WGR::padded * sizeof(double2) + (NY) * sizeof(double2) + 2 * WTD_KT * sizeof(double);
+template <class GR>
+__global__ void __launch_bounds__(WTD_SEP_NT) k_sep_rows(const double2 *__restrict__ in, double2 *lap, double2 *dy, const double *wa,
+                                                        const double *wb, int nfa, int nrows, const double2 *gtw_y, const double *gk)
+{
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    double2 *B = (double2 *)smem_raw, *W = B + GR::padded, *tw = W + GR::padded;
+    double *k2 = (double *)(tw + NY), *k1 = k2 + WTD_KT;   /* k_y of a digit-reversed position, Nyquist kept / zeroed */
+    constexpr int R = GR::N0, NP = GR::ntot;
+    for (int t = threadIdx.x; t < NY; t += WTD_SEP_NT) {
+        tw[t] = gtw_y[t];
+        k2[t] = gk[WTD_KT + t];
+        k1[t] = gk[4 * WTD_KT + t];
+    }
+    const int r0 = blockIdx.x * R, here = (nrows - r0 < R ? nrows - r0 : R) * NY;
+    const size_t base = (size_t)r0 * NY;                    /* rows of all fields are contiguous */
+    for (int p = threadIdx.x; p < NP; p += WTD_SEP_NT) {
+        double2 z = p < here ? in[base + p] : make_double2(0.0, 0.0);
+        if (wa && p < here) {
+            const int r = p / NY, f = (r0 + r) / NX, x = r0 + r - f * NX;
+            const double a = (f < nfa ? wa : wb)[(size_t)x * NY + (p - r * NY)];
+            z = make_double2(z.x * a, z.y * a);
+        }
+        B[GR::off(p)] = z;
+    }
+    __syncthreads();
+    fft_axis_fwd<GR, 1, 0, NY, 1>(B, 0, tw);
+    const double inv = 1.0 / (double)(NY);
+    if (dy) {
+        for (int p = threadIdx.x; p < NP; p += WTD_SEP_NT) {
+            const double k = k1[p % NY] * inv;
+            const double2 z = B[GR::off(p)];
+            W[GR::off(p)] = make_double2(-k * z.y, k * z.x);
+        }
+        __syncthreads();
+        fft_axis_inv<GR, 1, NY, 1>(W, 0, tw);
+        for (int p = threadIdx.x; p < here; p += WTD_SEP_NT) dy[base + p] = W[GR::off(p)];
+    }
+    if (lap) {
+        for (int p = threadIdx.x; p < NP; p += WTD_SEP_NT) {
+            const double k = k2[p % NY], sc = -(k * k) * inv;
+            const double2 z = B[GR::off(p)];
+            B[GR::off(p)] = make_double2(z.x * sc, z.y * sc);
+        }
+        __syncthreads();
+        fft_axis_inv<GR, 1, NY, 1>(B, 0, tw);
+        for (int p = threadIdx.x; p < here; p += WTD_SEP_NT) lap[base + p] = B[GR::off(p)];
+    }
+}
+#endif
+
 typedef Geo<NX, WTD_PXS, 1> WGXS;    /* WTD_PXS pencils along x */
 static constexpr size_t sep_planes_smem = 2 * (size_t)WGP::padded * sizeof(double2) + WGP::twtotal * sizeof(double2) + sizeof(KTab<WGP>);
 static constexpr size_t sep_pencils_smem = 2 * (size_t)WGXS::padded * sizeof(double2) + WGXS::twtotal * sizeof(double2) + sizeof(KTab<WGXS>);
@@ -300,6 +357,15 @@ static int big_derivs_sep(const double2 *in, int nf, double2 *lap, double2 *dx, 
                                     (int)cudaSharedmemCarveoutMaxShared));
         WTD_CU(cudaFuncSetAttribute(k_sep_pencils<WGXS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sep_pencils_smem)));
     const int nfa = nf / 2;
+#if CODEDIM == 2
+    if (sep_rows_smem <= WTD_SMEM_MAX && !dz) {
+        WTD_ONCE_PER_DEVICE(
+            WTD_CU(cudaFuncSetAttribute(k_sep_rows<WGR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sep_rows_smem)));
+        if (lap || dy)
+            k_sep_rows<WGR><<<(nf * NX + WGR::N0 - 1) / WGR::N0, WTD_SEP_NT, sep_rows_smem, st>>>(in, lap, dy, wa, wb, nfa, nf * NX,
+                                                                                               tw + NX, ktab);
+    } else
+#endif
     if (lap || dy || dz)
         k_sep_planes<WGP><<<nf * NX, WTD_SEP_NT, sep_planes_smem, st>>>(in, lap, dy, dz, wa, wb, nfa, tw + NX, ktab);
     if (lap || dx)
@@ -318,15 +384,6 @@ __global__ void k_c_to_real(const double2 *c, double *f, int n, double scale, in
     int i = threadIdx.x + blockIdx.x * blockDim.x;
     if (i < n) f[i] = accumulate ? f[i] + scale * c[i].x : scale * c[i].x;
 }
-/* tau = max(0, lap(rho)/2 - tau_tmp) from the staged laplacian (pca_dens.cu:275-290) */
-__global__ void k_tau_from_lap(const double2 *lap, double *tau, int n)
-{
-    int i = threadIdx.x + blockIdx.x * blockDim.x;
-    if (i >= n) return;
-    double t = 0.5 * lap[i].x - tau[i];
-    tau[i] = t < 0.0 ? 0.0 : t;
-}
-
 /* out (+)= scale * op(f) for a real field: which 0 = laplacian, 1..3 = d/dx, d/dy, d/dz.
  * stage holds 2N complex numbers of scratch. */
 static int big_real_deriv(const double *f, double *out, int which, double scale, int accumulate, double2 *stage,
@@ -362,32 +419,56 @@ static int big_filter_real(double *f, int nf, double mu, double T, double2 *stag
     return cudaGetLastError() == cudaSuccess ? WTD_OK : WTD_ERR_CUDA;
 }
 
+/* two real fields (of the two spins) at once through the transforms: to complex, back, and tau */
+__global__ void k_real2_to_c(const double *f0, const double *f1, double2 *c, int n)
+{
+    const int i = threadIdx.x + blockIdx.x * blockDim.x;
+    if (i < n) c[i] = make_double2(f0[i], 0.0);
+    else if (i < 2 * n) c[i] = make_double2(f1[i - n], 0.0);
+}
+__global__ void k_c_to_real2(const double2 *c, double *f0, double *f1, int n, double scale, int accumulate)
+{
+    const int i = threadIdx.x + blockIdx.x * blockDim.x;
+    if (i >= 2 * n) return;
+    double *f = i < n ? f0 + i : f1 + (i - n);
+    *f = accumulate ? *f + scale * c[i].x : scale * c[i].x;
+}
+__global__ void k_tau2_from_lap(const double2 *lap, double *tau0, double *tau1, int n)
+{
+    const int i = threadIdx.x + blockIdx.x * blockDim.x;
+    if (i >= 2 * n) return;
+    double *tau = i < n ? tau0 + i : tau1 + (i - n);
+    const double t = 0.5 * lap[i].x - *tau;
+    *tau = t < 0.0 ? 0.0 : t;
+}
+
 /* tau of both spins on a large lattice */
 static int big_tau(double *dens, double2 *stage, const double2 *tw, const double *kt, cudaStream_t st)
 {
     constexpr int N = NX * NY * NZ;
-    const int nb = (N + 255) / 256;
-    for (int s = 0; s < 2; s++) {
-        k_real_to_c<<<nb, 256, 0, st>>>(dens + (s == 0 ? 2 : 7) * (size_t)N, stage, N);
-        int r = big_derivs(stage, 1, stage, NULL, NULL, NULL, tw, kt, st);
-        if (r) return r;
-        k_tau_from_lap<<<nb, 256, 0, st>>>(stage, dens + (s == 0 ? 3 : 8) * (size_t)N, N);
-    }
+    const int nb = (2 * N + 255) / 256;
+    k_real2_to_c<<<nb, 256, 0, st>>>(dens + 2 * (size_t)N, dens + 7 * (size_t)N, stage, N);
+    WTD_TRY(big_derivs(stage, 2, stage, NULL, NULL, NULL, tw, kt, st));
+    k_tau2_from_lap<<<nb, 256, 0, st>>>(stage, dens + 3 * (size_t)N, dens + 8 * (size_t)N, N);
     return cudaGetLastError() == cudaSuccess ? WTD_OK : WTD_ERR_CUDA;
 }
 
 /* variable mass on a large lattice: CF_NA/NB = lap(alpha)/4, CF_CJA/CJB = -div(A)/2
- * (pca_kernels.cu:778-795), from the CF_ALA.. / CF_AAX.. rows already in cf */
+ * (pca_kernels.cu:778-795), from the CF_ALA.. / CF_AAX.. rows already in cf; both spins at once,
+ * in place in the staging buffer */
 static int big_prep_var(double *cf, double2 *stage, const double2 *tw, const double *kt, cudaStream_t st)
 {
     constexpr size_t N = (size_t)NX * NY * NZ;
-    for (int s = 0; s < 2; s++) {
-        WTD_TRY(big_real_deriv(cf + (s == 0 ? CF_ALA : CF_ALB) * N, cf + (s == 0 ? CF_NA : CF_NB) * N, 0, 0.25, 0, stage, tw, kt, st));
-        for (int d = 0; d < 3; d++)
-            WTD_TRY(big_real_deriv(cf + ((s == 0 ? CF_AAX : CF_ABX) + d) * N, cf + (s == 0 ? CF_CJA : CF_CJB) * N, d + 1, -0.5,
-                                   d > 0, stage, tw, kt, st));
+    const int nb = (int)((2 * N + 255) / 256);
+    k_real2_to_c<<<nb, 256, 0, st>>>(cf + CF_ALA * N, cf + CF_ALB * N, stage, (int)N);
+    WTD_TRY(big_derivs(stage, 2, stage, NULL, NULL, NULL, tw, kt, st));
+    k_c_to_real2<<<nb, 256, 0, st>>>(stage, cf + CF_NA * N, cf + CF_NB * N, (int)N, 0.25, 0);
+    for (int d = 0; d < CODEDIM; d++) {
+        k_real2_to_c<<<nb, 256, 0, st>>>(cf + (CF_AAX + d) * N, cf + (CF_ABX + d) * N, stage, (int)N);
+        WTD_TRY(big_derivs(stage, 2, NULL, d == 0 ? stage : NULL, d == 1 ? stage : NULL, d == 2 ? stage : NULL, tw, kt, st));
+        k_c_to_real2<<<nb, 256, 0, st>>>(stage, cf + CF_CJA * N, cf + CF_CJB * N, (int)N, -0.5, d > 0);
     }
-    return WTD_OK;
+    return cudaGetLastError() == cudaSuccess ? WTD_OK : WTD_ERR_CUDA;
 }
 
 #endif

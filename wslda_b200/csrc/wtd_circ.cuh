@@ -335,4 +335,28 @@ __device__ __forceinline__ void circ_lap(const C *src, C *dst)
     }
 }
 
+/* dst (padded, shared memory) = laplacian of the component y stored in natural order (global
+ * memory; a 3D lattice's lines are read in whole segments of the fastest axis or from L1) */
+template <class CG, typename C>
+__device__ __forceinline__ void circ_lap_from(const C *y, C *dst)
+{
+    typedef typename std::remove_const<decltype(y[0].x)>::type RC;
+    typedef typename std::remove_const<RC>::type R;
+#pragma unroll 1
+    for (int r0 = 0; r0 < CG::total; r0 += blockDim.x) {
+        const CircLine<CG> L(r0 + threadIdx.x);
+        R v[CG::nmax];
+        if (L.on)
+            circ_axis<CG>(L.ax, [&](auto A) {
+                constexpr int AX = decltype(A)::value, n = CG::n(AX);
+                R l[n];
+                circ::MemLine<R> f{(const R *)y + 2 * L.pb + L.c, 2 * L.ps};
+                circ::line_from<circ::LAP, AX, n>(f, l);
+#pragma unroll
+                for (int j = 0; j < n; j++) v[j] = l[j];
+            });
+        circ_store<CG, false>((R *)dst, L, v, r0);
+    }
+}
+
 #endif

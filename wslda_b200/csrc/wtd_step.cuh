@@ -158,14 +158,19 @@ template <class G, typename TC, bool VAR> struct FusedCfg {
      * once; the others run 256 threads */
     static constexpr int lines = (CG::total + 31) / 32 * 32;
     static constexpr int pts = (G::ntot + 31) / 32 * 32;
+    /* 3D with constant mass: a component has more lines than the block has threads, and they are
+     * read from global memory (L2, L1) in rounds instead of from a staged copy: pass A of 895 states
+     * of 12^3 126 -> 114 us.  With variable mass, which reads every line three times, the copy is
+     * faster (146 us against 160 us, 447 states) */
+    static constexpr bool from_global = circ && CG::dims == 3 && !VAR;
     static constexpr int threads = !circ ? (G::ntot >= 512 ? 512 : pts)
                                  : CG::nmax > 32 ? (lines < 128 ? 128 : lines > 256 ? 256 : lines)
                                  : pts < 256 ? (pts > lines ? pts : lines > 256 ? 256 : lines) : 256;
     /* CTAs per SM asked of the register allocator */
     static constexpr int minb = !circ ? (sizeof(TC) == 4 && threads == 512 ? 2 : 1)
                               : CG::nmax > (sizeof(TC) == 4 ? 64 : 48) || (VAR && CG::nmax > 16) ? 1 : 2;
-    static constexpr bool inplace = circ && !VAR && CG::total <= threads;
-    static constexpr int nbuf(bool grad) { return !circ ? (VAR ? 4 : grad ? 3 : 2) : inplace && !grad ? 2 : 3; }
+    static constexpr bool inplace = circ && !VAR && !from_global && CG::total <= threads;
+    static constexpr int nbuf(bool grad) { return !circ ? (VAR ? 4 : grad ? 3 : 2) : (from_global || inplace) && !grad ? 2 : 3; }
 };
 
 template <class G, typename TC, bool VAR, bool GRAD> struct FusedSmem {
@@ -207,7 +212,10 @@ __device__ __forceinline__ double hpsi_const(const TY *yu, const TY *yv, typenam
     typedef typename Cfg::Lay Lay;
     constexpr int N = G::ntot;
     const uint64_t pol = l2_policy_keep();
-    if constexpr (Cfg::circ && !Cfg::inplace) {
+    if constexpr (Cfg::from_global) {
+#pragma unroll 1
+        for (int comp = 0; comp < 2; comp++) circ_lap_from<Lay>((const C *)(comp ? yv : yu), comp ? BV : BU);
+    } else if constexpr (Cfg::circ && !Cfg::inplace) {
 #pragma unroll 1
         for (int comp = 0; comp < 2; comp++) {
             const TY *y = comp ? yv : yu;
@@ -516,9 +524,10 @@ __device__ __forceinline__ void dens_gradients(double *ds, const TY *ysrc, typen
             const int nax = L.ax == 0 ? Lay::n(0) : L.ax == 1 ? Lay::n(1) : Lay::n(2);
             int st = L.st;
             asm volatile("" : "+r"(st));
+            const TC *so = s + (L.base ^ 1);
 #pragma unroll
             for (int j = 0; j < Lay::nmax; j++) {
-                const double o = j < nax ? (double)s[(L.base ^ 1) + j * st] : 0.0;
+                const double o = j < nax ? (double)so[j * st] : 0.0;
                 const double a = (L.c ? 1.0 : -1.0) * o * (double)d[j];
                 const double b = a + __shfl_xor_sync(0xffffffffu, a, 1);
                 if (L.on && L.c == 0 && j < nax) red_keep(dj + (size_t)j * L.ps, jsgn * b * fw, pol);

@@ -143,10 +143,12 @@ template <typename TY, typename TH, typename TC, int PASS, bool GRAD> struct Fus
     static constexpr size_t smem = FusedSmem<WG, TC, WTD_VAR, GRAD>::bytes;
     static constexpr bool fits = smem <= WTD_SMEM_MAX && FusedSmem<WG, TC, WTD_VAR, GRAD>::fft_bytes <= WTD_SMEM_MAX;
     static constexpr bool wide = !Cfg::circ && WG::ntot >= 2048;
+    /* gradient passes on lines of more than 48 points apply two operators and would spill 700 bytes
+     * at two CTAs an SM: one (64^2 FP32, 8192 states: 3.8 -> 2.8 ms) */
     template <int BS> static auto kernel()
     {
         return wtd_fused_pass<WG, TY, TH, TC, WTD_NHIST, PASS, WTD_VAR, GRAD, BS,
-                              Cfg::circ || BS == 512 ? Cfg::minb : 1>;
+                              Cfg::circ ? (GRAD && Cfg::CG::nmax > 48 ? 1 : Cfg::minb) : BS == 512 ? Cfg::minb : 1>;
     }
     static constexpr int BS = Cfg::circ ? Cfg::threads : 512;
 };

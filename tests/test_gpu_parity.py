@@ -141,7 +141,7 @@ def test_c5_slda3d_small_s(has_gpu, monkeypatch, path):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("nwf", [2, 7, 130])
+@pytest.mark.parametrize("nwf", [7, 8, 130])
 def test_t3d_ragged_stream_path(has_gpu, nwf):
     """3D beyond one CTA with unequal axes (20 x 18 x 22: circulant lines with odd factors, 4 columns
     per block of the x kernels, a partial last group of states) in FP64"""

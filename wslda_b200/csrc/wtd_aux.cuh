@@ -314,15 +314,15 @@ __global__ void __launch_bounds__(32 * WTD_RED_W) wtd_limited_after(const double
     }
 #pragma unroll
     for (int j = 0; j < 4; j++) part[j][w][lane] = s[j];
-    __syncthreads();
-    if (!on) return;
-    if (w > 0) {
-        /* the eight words of tau and j are zero in this half step */
+    /* the eight words of tau and j are zero in this half step; stored ahead of the barrier, after
+     * which warp 0's functional may read them (SLDAE does) */
+    if (on && w > 0) {
         const int z = w - 1;                                   /* 0..6 of tau_a, j_a, tau_b, j_b */
         dens[(size_t)(z < 4 ? 3 + z : 4 + z) * N + i] = 0.0;
         if (w == 1) dens[11 * N + i] = 0.0;
-        return;
     }
+    __syncthreads();
+    if (!on || w > 0) return;
 #pragma unroll
     for (int k = 1; k < WTD_RED_W; k++)
 #pragma unroll

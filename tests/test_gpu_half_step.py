@@ -49,3 +49,47 @@ def test_half_step_without_gradients_clears_tau_before_the_functional(has_gpu, n
         return out
     for a, b in zip(run(False), run(True)):
         assert np.array_equal(a, b)
+
+
+@pytest.mark.gpu
+def test_stream_path_takes_more_than_65535_states(has_gpu):
+    """the state count is no grid extent limited to 65,535: 20 x 18 x 22 with 65,540 complex64 states
+    (50 GB), normalised from arbitrary norms, measured and stepped"""
+    import torch
+    from wslda_b200 import MIXED_H32, TDRun
+    from wslda_b200.projects import Project, make_potentials
+    proj, S = Project("t3d_ragged"), 65540
+    if torch.cuda.mem_get_info()[0] < 70e9:
+        pytest.skip("needs 70 GB of free device memory")
+    r = TDRun(proj, S, precision=MIXED_H32)
+    states, dens = _device(r, (2, S, r.N), "<c8")
+    g = torch.Generator(device="cuda")
+    g.manual_seed(5)
+    parts = [(a, min(a + 4096, S)) for a in range(0, S, 4096)]
+
+    def norms():
+        return torch.cat([(states[:, a:b].abs() ** 2).sum(dim=(0, 2), dtype=torch.float64) for a, b in parts]) * proj.dv
+    for a, b in parts:
+        states[:, a:b] = torch.randn((2, b - a, r.N), dtype=torch.complex64, device="cuda", generator=g)
+    # the component that a state adds to the densities is its small one, so that 65,540 states on
+    # 7,920 points stay dilute (0.04 per point and spin)
+    occ = (np.arange(S) % 2 == 0).astype(float)
+    states[0, 0::2] *= 0.1
+    states[1, 1::2] *= 0.1
+    r.setup_fields(make_potentials(proj), occ, proj.params)
+    torch.cuda.synchronize()
+    for call in (r.initial_measurement, lambda: r.steps(1)):
+        call()
+        r.sync()
+        n = norms()
+        assert float((n - 1.0).abs().max()) < 1e-6
+        # rho_a = sum f |u|^2, rho_b = sum (1 - f) |v|^2, over all the states
+        f = torch.tensor(occ, device="cuda")
+        want = torch.zeros(2, r.N, dtype=torch.float64, device="cuda")
+        for a, b in parts:
+            want[0] += ((states[0, a:b].abs() ** 2).double() * f[a:b, None]).sum(0)
+            want[1] += ((states[1, a:b].abs() ** 2).double() * (1.0 - f[a:b, None])).sum(0)
+        for k, off in ((0, 2), (1, 7)):
+            got = dens[off * r.N:(off + 1) * r.N]
+            assert float(torch.linalg.vector_norm(got - want[k]) / torch.linalg.vector_norm(want[k])) < 1e-6
+    r.close()

@@ -650,7 +650,7 @@ template <typename TY, typename TH, typename TC> struct Stream {
     }
     template <int PASS> static int abm(wtd_ctx *c, const StepArgs &a)
     {
-        k3s_abm<TY, TH, TC, WTD_NHIST, PASS><<<dim3(2 * S3::ACH, c->S), S3::AT, 0, c->st>>>(a, (const C *)c->kbuf, c->sc, c->part);
+        k3s_abm<TY, TH, TC, WTD_NHIST, PASS><<<S3::states_grid(c->S), S3::AT, 0, c->st>>>(a, (const C *)c->kbuf, c->sc, c->part);
         WTD_LAUNCHED(c);
         return PASS == 3 ? WTD_OK : sum(c, 2 * S3::ACH, c->sc, 1);
     }
@@ -701,7 +701,7 @@ template <typename TY, typename TH, typename TC> struct Stream {
     }
     static int rescale(wtd_ctx *c)
     {
-        k3s_rescale<TY><<<dim3(2 * S3::ACH, c->S), S3::AT, 0, c->st>>>((TY *)c->y, c->sc, c->S);
+        k3s_rescale<TY><<<S3::states_grid(c->S), S3::AT, 0, c->st>>>((TY *)c->y, c->sc, c->S);
         WTD_LAUNCHED(c);
         k3s_fill<<<(c->S + 255) / 256, 256, 0, c->st>>>(c->sc, 1.0, c->S);
         WTD_LAUNCHED(c);

@@ -43,8 +43,15 @@ struct S3 {
     static constexpr int XL = 2 * QB;                       /* threads of one (state, component) */
     static constexpr int XS = 64 / XL;                      /* states in flight (whole warps for any QB) */
     static constexpr unsigned XM = 2 * XL >= 32 ? 0xffffffffu : (1u << (2 * XL)) - 1u;   /* lanes of k3s_dens_x */
-    /* elements per CTA of k3s_abm along one component */
+    /* elements per CTA of k3s_abm along one component; 2 ACH CTAs a state */
     static constexpr int AT = 256, AE = 4, ACH = (N + AT * AE - 1) / (AT * AE);
+    /* grid of 2 ACH CTAs for each of S states: the states over y and z, whose extents stop at 65535
+     * (all in x, with a division per CTA, took 1% of a step in the all-FP32 form) */
+    static dim3 states_grid(int S)
+    {
+        const unsigned z = ((unsigned)S + 65534u) / 65535u;
+        return dim3(2 * ACH, ((unsigned)S + z - 1) / z, z);
+    }
 };
 
 /* ---- shared memory of the plane kernel: coefficient planes (variable mass), then per state in
@@ -335,7 +342,8 @@ __global__ void __launch_bounds__(S3::AT) k3s_abm(StepArgs a, const typename cpl
     typedef typename cplx<TC>::t C;
     constexpr int N = S3::N, AT = S3::AT, AE = S3::AE;
     __shared__ double red[80];
-    const int ch = blockIdx.x % S3::ACH, comp = blockIdx.x / S3::ACH, n = blockIdx.y;
+    const int ch = blockIdx.x % S3::ACH, comp = blockIdx.x / S3::ACH, n = blockIdx.y + gridDim.y * blockIdx.z;
+    if (n >= a.S) return;
     const size_t fb = ((size_t)comp * a.S + n) * N;
     const int i0 = ch * (AT * AE) + threadIdx.x;
     const bool haveH = PASS == 1 || PASS == 3 || (PASS == 0 && !a.fk_given);
@@ -411,7 +419,8 @@ template <typename TY>
 __global__ void __launch_bounds__(S3::AT) k3s_rescale(TY *Y, const double *__restrict__ sc, int S)
 {
     constexpr int N = S3::N;
-    const int ch = blockIdx.x % S3::ACH, comp = blockIdx.x / S3::ACH, n = blockIdx.y;
+    const int ch = blockIdx.x % S3::ACH, comp = blockIdx.x / S3::ACH, n = blockIdx.y + gridDim.y * blockIdx.z;
+    if (n >= S) return;
     const size_t fb = ((size_t)comp * S + n) * N;
     const double s = sc[n];
 #pragma unroll

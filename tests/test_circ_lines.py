@@ -1,10 +1,10 @@
 """Compile-time coefficients of the folded lines (wtd_circ.cuh) against their defining sums in
 80-bit arithmetic, on the CPU.
 
-A coefficient is k0^(2 or 1) times a combination of the operator's kernel t(d) on N points, k0 the
-double 2 pi / L.  It is rounded once, so it lies within half a unit in the last place (2^-53
-relative) of the exact value; the sum of N terms of at most N^2/4 in 80 bits is good to
-N 2^-64 max |t| k0^p, which is added to the bound.
+A coefficient is a combination of the operator's kernel t(d) on N points, with the doubles k_q and
+k_q^2 of the transforms' tables as its symbol.  It is rounded once, so it lies within half a unit in
+the last place (2^-53 relative) of the exact value; the mean of N terms in 80 bits is good to
+N 2^-64 max |symbol|, which is added to the bound.
 """
 import os
 import subprocess
@@ -33,13 +33,15 @@ static double worst = 0.0;
 static int count = 0;
 
 /* (1/N) sum_q of the operator's symbol times e^{2 pi i q d/N}, Nyquist mode zeroed in the derivative */
+static double k0;      /* 2 pi / L of the axis */
 static Q exact_t(int op, int N, int d)
 {
     Q s = 0;
     for (int q = -N / 2; q < N / 2; q++) {
         const Q a = 2 * PIQ * (((Q)q * d) - N * roundl((Q)q * d / N)) / N;
-        if (op == circ::LAP) s -= (Q)q * q * cosl(a);
-        else if (q != -N / 2) s -= (Q)q * sinl(a);
+        const double k = k0 * (double)q, k2 = k * k;
+        if (op == circ::LAP) s -= (Q)k2 * cosl(a);
+        else if (q != -N / 2) s -= (Q)k * sinl(a);
     }
     return s / N;
 }
@@ -53,12 +55,11 @@ static Q exact_b(int op, int N, int n, bool skew, int d)
 }
 template <int OP, int AX, int N, int n, bool SKEW, bool EV, int j, int k> static void one()
 {
-    const double L = AX == 0 ? LX : AX == 1 ? LY : LZ, k0 = 2.0 * 3.14159265358979323846 / L;
+    k0 = 2.0 * 3.14159265358979323846 / (AX == 0 ? LX : AX == 1 ? LY : LZ);
     const Q a = exact_b(OP, N, n, SKEW, j - k), b = exact_b(OP, N, n, SKEW, j + k);
     const bool self = EV ? circ::self_even(n, SKEW, k) : circ::self_odd(n, SKEW, k);
-    const Q sc = OP == circ::LAP ? (Q)k0 * k0 : (Q)k0;
-    const Q want = (self ? a : EV ? (a + b) / 2 : (a - b) / 2) * sc;
-    const Q bound = fabsl(want) * 0x1p-53L + N * 0x1p-64L * (OP == circ::LAP ? (Q)N * N / 4 : (Q)N / 2) * sc;
+    const Q want = self ? a : EV ? (a + b) / 2 : (a - b) / 2, kmax = k0 * N / 2;
+    const Q bound = fabsl(want) * 0x1p-53L + N * 0x1p-64L * (OP == circ::LAP ? kmax * kmax : kmax);
     const double got = circ::Coef<OP, AX, N, n, SKEW, EV, j, k>::value;
     const double e = (double)(fabsl((Q)got - want) / bound);
     if (!(e <= worst)) worst = e;

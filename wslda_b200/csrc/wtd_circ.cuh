@@ -30,7 +30,7 @@ namespace circ {
 /* The coefficients are formed at compile time as unevaluated sums of two doubles (Dekker 1971, Numer.
  * Math. 18) and rounded once.  They are the same in every step, so their errors add up coherently
  * over a run: formed in plain doubles they made up nearly all of the operators' error (laplacian
- * of 12 points: 1.8e-16 of 1.9e-16 relative, rounded once 0.8e-16 of 1.4e-16). */
+ * of 12 points: 1.8e-16 of 1.9e-16 relative, rounded once 0.9e-16 of 1.4e-16). */
 struct dd {
     double h, l;
 };
@@ -95,47 +95,51 @@ constexpr dd cos_pi(int d, int n)
 
 enum { LAP = 0, DER = 1 };
 
-/* kernel of the operator on n points (n even) in units of the wave-number spacing: laplacian
- * t(d) = (1/n) sum_q -q^2 e^{2 pi i q d/n}, derivative t(d) = (1/n) sum_q i q e^{2 pi i q d/n}
- * without q = n/2 (closed forms), 0 <= d < n */
-template <int OP> constexpr dd kernel(int n, int d)
+/* kernel of the operator along axis AX on N points (N even) from the symbol that the transforms
+ * apply, k_q = (2 pi / L) q and its square as doubles, Nyquist mode zeroed in the derivative:
+ * laplacian t(d) = (1/N) sum_q -k_q^2 e^{2 pi i q d/N}, derivative t(d) = (1/N) sum_q i k_q
+ * e^{2 pi i q d/N} */
+template <int OP, int AX> constexpr double symbol(int q)
 {
-    const double sgn = (d % 2) ? -0.5 : 0.5;
-    if (OP == LAP) {
-        if (d == 0) return neg(quo(dd{(double)n * n + 2.0, 0.0}, dd{12.0, 0.0}));
-        const dd s = sin_pi(d, n);
-        return quo(dd{-sgn, 0.0}, mul(s, s));
-    }
-    return d == 0 ? dd{0.0, 0.0} : scl(quo(cos_pi(d, n), sin_pi(d, n)), sgn);
+    const double k = 2.0 * PI2.h / (AX == 0 ? (double)(LX) : AX == 1 ? (double)(LY) : (double)(LZ)) * (double)q;
+    return OP == LAP ? -(k * k) : -k;
 }
 /* kernel of the circulant block of n points inside a line of N: 2^-l sum_s t(d + s n), N = 2^l n,
  * from that of 2 n points */
-template <int OP, int N, int n> struct Cyc {
+template <int OP, int AX, int N, int n> struct Cyc {
     dd t[n];
     constexpr Cyc() : t()
     {
         if constexpr (n == N) {
-            for (int d = 0; 2 * d <= n; d++) t[d] = kernel<OP>(n, d);
-            for (int d = 1; 2 * d < n; d++) t[n - d] = OP == LAP ? t[d] : neg(t[d]);
+            dd w[N] = {};   /* cos or sin (2 pi m / N) */
+            for (int m = 0; 2 * m <= N; m++) w[m] = OP == LAP ? cos_pi(2 * m, N) : sin_pi(2 * m, N);
+            for (int m = 1; 2 * m < N; m++) w[N - m] = OP == LAP ? w[m] : neg(w[m]);
+            for (int d = 0; 2 * d <= N; d++) {
+                dd s{0.0, 0.0};
+                for (int q = N / 2 - 1; q > 0; q--) s = add(s, scl(w[q * d % N], 2.0 * symbol<OP, AX>(q)));
+                if (OP == LAP) s = add(s, scl(w[N / 2 * d % N], symbol<OP, AX>(N / 2)));
+                t[d] = quo(s, dd{(double)N, 0.0});
+            }
+            for (int d = 1; 2 * d < N; d++) t[N - d] = OP == LAP ? t[d] : neg(t[d]);
         } else {
-            const Cyc<OP, N, 2 * n> p;
+            const Cyc<OP, AX, N, 2 * n> p;
             for (int d = 0; d < n; d++) t[d] = scl(add(p.t[d], p.t[d + n]), 0.5);
         }
     }
 };
 /* kernel of the skew block of n points (the m half of the circulant of 2 n points) */
-template <int OP, int N, int n> struct Skw {
+template <int OP, int AX, int N, int n> struct Skw {
     dd t[n];
     constexpr Skw() : t()
     {
-        const Cyc<OP, N, 2 * n> p;
+        const Cyc<OP, AX, N, 2 * n> p;
         for (int d = 0; d < n; d++) t[d] = scl(add(p.t[d], neg(p.t[d + n])), 0.5);
     }
 };
 /* either, at any d: periodic, or antiperiodic where skew */
-template <int OP, int N, int n, bool SKEW> constexpr dd tk(int d)
+template <int OP, int AX, int N, int n, bool SKEW> constexpr dd tk(int d)
 {
-    constexpr typename std::conditional<SKEW, Skw<OP, N, n>, Cyc<OP, N, n>>::type T;
+    constexpr typename std::conditional<SKEW, Skw<OP, AX, N, n>, Cyc<OP, AX, N, n>>::type T;
     const int m = ((d % (2 * n)) + 2 * n) % (2 * n), r = m % n;
     return SKEW && m >= n ? neg(T.t[r]) : T.t[r];
 }
@@ -147,19 +151,11 @@ constexpr int n_odd(int n, bool skew) { return skew ? n / 2 : (n - 1) / 2; }
 constexpr bool self_even(int n, bool skew, int k) { return k == 0 || (!skew && 2 * k == n); }
 constexpr bool self_odd(int n, bool skew, int k) { return skew && 2 * k == n; }
 
-/* wave-number spacing 2 pi / L of the lattice axis AX (the double that the wave numbers of the
- * transforms are multiples of), to the operator's order */
-template <int OP, int AX> constexpr dd axis_scale()
-{
-    const double k = 2.0 * PI2.h / (AX == 0 ? (double)(LX) : AX == 1 ? (double)(LY) : (double)(LZ));
-    return OP == LAP ? two_prod(k, k) : dd{k, 0.0};
-}
-
 /* coefficient from even input k (EV) or odd input k to output row j */
 template <int OP, int AX, int N, int n, bool SKEW, bool EV, int j, int k> struct Coef {
     static constexpr bool self = EV ? self_even(n, SKEW, k) : self_odd(n, SKEW, k);
-    static constexpr dd a = tk<OP, N, n, SKEW>(j - k), b = tk<OP, N, n, SKEW>(j + k);
-    static constexpr double value = mul(self ? a : scl(add(a, EV ? b : neg(b)), 0.5), axis_scale<OP, AX>()).h;
+    static constexpr dd a = tk<OP, AX, N, n, SKEW>(j - k), b = tk<OP, AX, N, n, SKEW>(j + k);
+    static constexpr double value = self ? a.h : scl(add(a, EV ? b : neg(b)), 0.5).h;
 };
 
 template <int OP, int AX, int N, int n, bool SKEW, bool EV, int j, int k, int K1, typename R>

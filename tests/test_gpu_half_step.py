@@ -93,3 +93,29 @@ def test_stream_path_takes_more_than_65535_states(has_gpu):
             got = dens[off * r.N:(off + 1) * r.N]
             assert float(torch.linalg.vector_norm(got - want[k]) / torch.linalg.vector_norm(want[k])) < 1e-6
     r.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("name,nwf,prec", [("t3d_ragged", 9, 2), ("c3_aslda3d", 8, 1), ("c3_aslda3d", 8, 2), ("c5_slda3d", 4, 2)])
+def test_densities_are_those_of_the_returned_states(has_gpu, name, nwf, prec):
+    """the complex64 forms sum the densities of the states that the call leaves, not of states rounded
+    once more afterwards: rho and nu formed from the returned states agree to FP64 rounding of sums of
+    nwf terms"""
+    from wslda_b200 import TDRun
+    proj, d = inputs(name, nwf)
+    N = proj.numel
+    r = TDRun(name, nwf, precision=prec)
+    r.setup(d["states"], d["pots"], d["occ"], d["params"], d["extra"])
+    for call in (r.initial_measurement, lambda: r.steps(2), lambda: r.steps(1)):
+        call()
+        y, dens = r.states().reshape(2, nwf, N), r.densities()
+        f = np.asarray(d["occ"])[:, None]
+        u, v = y[0], y[1]
+        nu = ((u * v.conj()) * (1.0 - 2.0 * f) * 0.5).sum(0)
+        got = dens[:2 * N].view(np.complex128)
+        # relative to sum |u v|, which the signed sum nu cancels from
+        scale = np.sqrt(((np.abs(u) * np.abs(v) * 0.5).sum(0) ** 2).sum())
+        assert np.linalg.norm(got - nu) < 1e-14 * scale
+        for want, off in (((np.abs(u) ** 2 * f).sum(0), 2), ((np.abs(v) ** 2 * (1.0 - f)).sum(0), 7)):
+            assert np.linalg.norm(dens[off * N:(off + 1) * N] - want) < 1e-14 * np.linalg.norm(want)
+    r.close()

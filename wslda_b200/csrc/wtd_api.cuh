@@ -227,7 +227,7 @@ static int run_pass(wtd_ctx *c, int pass, bool grad)
 }
 
 static int line_pass(wtd_ctx *c, int pass, bool grad, const StepArgs *given = NULL);
-static int stream_pass(wtd_ctx *c, int pass, bool grad);
+static int stream_pass(wtd_ctx *c, int pass, bool grad, bool final = false);
 static int stream_coef_var(wtd_ctx *c);
 
 /* f1 = (H - <H>) psi of the current state and its quasiparticle energies, as the reference
@@ -642,9 +642,9 @@ template <typename TY, typename TH, typename TC> struct Stream {
     typedef S3XSmem<TC, WTD_VAR> XS;
     typedef S3DensSmem<TC> DS;
 
-    static int sum(wtd_ctx *c, int np, double *out, int norm, double *nrm_out = NULL)
+    static int sum(wtd_ctx *c, int np, double *out, int norm)
     {
-        k3s_sum<<<(c->S + 3) / 4, 128, 0, c->st>>>(c->part, np, c->S, out, norm, nrm_out);
+        k3s_sum<<<(c->S + 3) / 4, 128, 0, c->st>>>(c->part, np, c->S, out, norm, c->sc);
         WTD_LAUNCHED(c);
         return WTD_OK;
     }
@@ -669,19 +669,21 @@ template <typename TY, typename TH, typename TC> struct Stream {
         constexpr size_t N = S3::N;
         return c->dslot + (which > 0 ? (size_t)c->gpt * 4 * N : 0) + (which > 1 ? (size_t)c->gpl * 6 * N : 0);
     }
-    static int pass(wtd_ctx *c, int p, bool grad)
+    /* final: the last half step of a call, whose states the caller sees */
+    static int pass(wtd_ctx *c, int p, bool grad, bool final)
     {
         const StepArgs a = make_args(c);
         const TY *y = (const TY *)a.y;
         if (p == 1 || p == 3 || (p == 0 && !a.fk_given)) {
-            k3s_plane_h<TY, TC, WTD_VAR><<<c->p1grid, S3::LT * PS::NS, PS::bytes, c->st>>>(y, (C *)c->kbuf, c->cf, c->sc, c->S);
+            k3s_plane_h<TY, TC, WTD_VAR><<<c->p1grid, S3::LT * PS::NS, PS::bytes, c->st>>>(y, (C *)c->kbuf, c->cf, c->S);
             WTD_LAUNCHED(c);
-            k3s_x_h<TY, TC, WTD_VAR><<<c->xgrid, 2 * S3::XL * XS::NS, XS::bytes, c->st>>>(y, (C *)c->kbuf, c->cf, c->sc, c->part, c->S);
+            k3s_x_h<TY, TC, WTD_VAR><<<c->xgrid, 2 * S3::XL * XS::NS, XS::bytes, c->st>>>(y, (C *)c->kbuf, c->cf, c->part, c->S);
             WTD_LAUNCHED(c);
             WTD_TRY(sum(c, 2 * S3::NQB, c->qpe, 0));
         }
         WTD_TRY(p == 0 ? abm<0>(c, a) : p == 1 ? abm<1>(c, a) : p == 2 ? abm<2>(c, a) : abm<3>(c, a));
         if (p == 3) return WTD_OK;
+        if (final) WTD_TRY(rescale(c));
         return dens(c, c->wcnt, grad);
     }
     /* density sums of the current states with per-state weights w */
@@ -786,11 +788,11 @@ static size_t stream_part_words(const wtd_ctx *c) { return (size_t)c->S * 2 * (S
 
 /* one half step's kernels (pass 0: H y_k + predictor, 1: H y_pred + corrector, 2: norms and
  * densities, 3: f_k only), timed like the fused passes when timing is on */
-static int stream_pass(wtd_ctx *c, int pass, bool grad)
+static int stream_pass(wtd_ctx *c, int pass, bool grad, bool final)
 {
     const bool timed = c->timing && pass < 2 && c->nev[pass] < 4096;
     if (timed) cudaEventRecord(c->ev[pass][0][c->nev[pass]], c->st);
-    const int r = stream_form(c, [&](auto s) { return decltype(s)::pass(c, pass, grad); });
+    const int r = stream_form(c, [&](auto s) { return decltype(s)::pass(c, pass, grad, final); });
     if (timed) {
         cudaEventRecord(c->ev[pass][1][c->nev[pass]], c->st);
         c->nev[pass]++;
@@ -835,7 +837,7 @@ static int stream_step(wtd_ctx *c, bool last)
     WTD_TRY(stream_pass(c, 0, var));
     WTD_TRY(stream_after(c, var, c->it + 1));
     const bool g = var || last;
-    WTD_TRY(stream_pass(c, 1, g));
+    WTD_TRY(stream_pass(c, 1, g, last));
     WTD_TRY(stream_after(c, g, c->it + 1));
     c->head = (c->head + WTD_NHIST - 1) % WTD_NHIST;
     c->fk_given = 0;
@@ -843,17 +845,10 @@ static int stream_step(wtd_ctx *c, bool last)
     return WTD_OK;
 }
 
-/* the states in place times their scale: what every call leaves behind */
-static int stream_rescale(wtd_ctx *c)
-{
-    return stream_form(c, [&](auto s) { return decltype(s)::rescale(c); });
-}
-
 static int stream_initial(wtd_ctx *c)
 {
-    WTD_TRY(stream_pass(c, 2, true));
-    WTD_TRY(stream_after(c, true, -1));
-    return stream_rescale(c);
+    WTD_TRY(stream_pass(c, 2, true, true));
+    return stream_after(c, true, -1);
 }
 
 static int stream_setup(wtd_ctx *c, int nsm)
@@ -865,9 +860,8 @@ static bool stream_fits(int) { return false; }
 static int stream_coef_var(wtd_ctx *) { return WTD_ERR_UNSUPPORTED; }
 static size_t stream_slot_words(const wtd_ctx *) { return 0; }
 static size_t stream_part_words(const wtd_ctx *) { return 0; }
-static int stream_pass(wtd_ctx *, int, bool) { return WTD_ERR_UNSUPPORTED; }
+static int stream_pass(wtd_ctx *, int, bool, bool) { return WTD_ERR_UNSUPPORTED; }
 static int stream_step(wtd_ctx *, bool) { return WTD_ERR_UNSUPPORTED; }
-static int stream_rescale(wtd_ctx *) { return WTD_ERR_UNSUPPORTED; }
 static int stream_initial(wtd_ctx *) { return WTD_ERR_UNSUPPORTED; }
 static int stream_setup(wtd_ctx *, int) { return WTD_ERR_UNSUPPORTED; }
 static int stream_subset(wtd_ctx *, const double *, double *) { return WTD_ERR_UNSUPPORTED; }
@@ -1610,7 +1604,7 @@ int wtd_steps(wtd_ctx *c, int nsteps)
     }
     if (c->stream) {
         for (int s = 0; s < nsteps; s++) WTD_TRY(stream_step(c, s == nsteps - 1));
-        return nsteps > 0 ? stream_rescale(c) : WTD_OK;
+        return WTD_OK;
     }
     if (c->line) {
         for (int s = 0; s < nsteps; s++) WTD_TRY(line_step(c, s == nsteps - 1));

@@ -6,7 +6,7 @@
  * registers (wtd_circ.cuh), so a half step is a chain of plain streaming kernels:
  *
  *   k3s_plane_h     one CTA per (component, x-plane, chunk of states): the (y, z) part of the
- *                   kinetic and current terms of H psi (pca_kernels.cu:233-391) into h;
+ *                   kinetic and current terms of H psi (pca_kernels.cu:233-391) into h, unscaled;
  *   k3s_x_h         one CTA per (block of (y, z) columns, chunk of states): h += the x-line part
  *                   and the local terms; partial sums of <psi|H|psi>;
  *   k3s_abm         elementwise: f = h - <H> psi, the ABM predictor or corrector
@@ -14,11 +14,13 @@
  *   k3s_dens_*      densities of the updated states (pca_dens.cu:13-338): nu and rho per point,
  *                   and on gradient half steps tau and j along the plane's and the x lines.
  *
- * The updated states are stored before their norm is known; the kernels that read them next
- * multiply by the state's scale 1/norm (k3s_norm), and wtd_steps ends with the states scaled in
- * place (k3s_rescale).  Precision forms as in the fused pass: TY storage of the states, TH of
- * the ABM history, TC of the derivatives; local terms, ABM sums, norms, <H> and density sums
- * are FP64.
+ * The updated states are stored before their norm is known.  What is formed from them next is
+ * linear in the state (h) or quadratic (<H>, densities), so those kernels work on the stored values
+ * and the state's scale 1/norm (k3s_sum) is taken in FP64 where the result is next used or summed.
+ * In the last half step of a call the states are scaled in place (k3s_rescale) before their
+ * densities are summed, which are then those of the states that the caller sees.  Precision forms
+ * as in the fused pass: TY storage of the states, TH of the ABM history, TC of the derivatives;
+ * local terms, ABM sums, norms, <H> and density sums are FP64.
  */
 #ifndef WTD_STREAM3D_CUH
 #define WTD_STREAM3D_CUH
@@ -68,8 +70,7 @@ template <typename TC, bool VAR> struct S3PlaneSmem {
 
 template <typename TY, typename TC, bool VAR>
 __global__ void __launch_bounds__(S3::LT * S3PlaneSmem<TC, VAR>::NS)
-k3s_plane_h(const TY *__restrict__ Y, typename cplx<TC>::t *__restrict__ K, const double *__restrict__ cf,
-            const double *__restrict__ sc, int S)
+k3s_plane_h(const TY *__restrict__ Y, typename cplx<TC>::t *__restrict__ K, const double *__restrict__ cf, int S)
 {
     typedef typename cplx<TC>::t C;
     typedef S3PlaneSmem<TC, VAR> SM;
@@ -101,11 +102,10 @@ k3s_plane_h(const TY *__restrict__ Y, typename cplx<TC>::t *__restrict__ K, cons
         if (t == 0 && n + NS * nch < S) prefetch_l2(Y + base + (size_t)NS * nch * N, NYZ * sizeof(TY));
         __syncthreads();
         if (act) {
-            const TC s = (TC)sc[n];
 #pragma unroll 8
             for (int i = t; i < NYZ; i += LT) {
                 const TY a = Y[base + i];
-                C z; z.x = a.x * s; z.y = a.y * s;
+                C z; z.x = a.x; z.y = a.y;
                 P[(i / NZ) * PITCH + i % NZ] = z;
             }
         }
@@ -211,8 +211,7 @@ template <int T> __device__ __forceinline__ void state_sync(int slot)
 
 template <typename TY, typename TC, bool VAR>
 __global__ void __launch_bounds__(2 * S3::XL * S3XSmem<TC, VAR>::NS)
-k3s_x_h(const TY *__restrict__ Y, typename cplx<TC>::t *K, const double *__restrict__ cf, const double *__restrict__ sc,
-        double *__restrict__ epart, int S)
+k3s_x_h(const TY *__restrict__ Y, typename cplx<TC>::t *K, const double *__restrict__ cf, double *__restrict__ epart, int S)
 {
     typedef typename cplx<TC>::t C;
     typedef S3XSmem<TC, VAR> SM;
@@ -269,14 +268,10 @@ k3s_x_h(const TY *__restrict__ Y, typename cplx<TC>::t *K, const double *__restr
         }
         if (act) {
             const TC *yr = (const TC *)Y + 2 * base + c;
-            const TC s = (TC)sc[n];
 #pragma unroll
             for (int x = 0; x < NX; x++) f[x] = yr[(size_t)2 * x * NYZ];
 #pragma unroll
-            for (int x = 0; x < NX; x++) {
-                f[x] *= s;
-                ((TC *)Yo)[2 * (x * QB + q) + c] = f[x];
-            }
+            for (int x = 0; x < NX; x++) ((TC *)Yo)[2 * (x * QB + q) + c] = f[x];
             if (VAR) {
                 circ::line_op<circ::DER, 0, NX>(f, l);
 #pragma unroll
@@ -320,20 +315,21 @@ k3s_x_h(const TY *__restrict__ Y, typename cplx<TC>::t *K, const double *__restr
     }
 }
 
-/* out[n] = DV sum of the np partial sums of state n (norm: 1 / sqrt of it); one warp per state,
- * fixed order */
-__global__ void __launch_bounds__(128) k3s_sum(const double *part, int np, int S, double *out, int norm, double *nrm_out)
+/* DV sum of the np partial sums of state n, one warp per state, fixed order.  norm: out[n] = 1 / sqrt of
+ * it, the state's scale; else out[n] = it times the square of the scale sc[n] (the partial sums of
+ * <H> are of the stored states) */
+__global__ void __launch_bounds__(128) k3s_sum(const double *part, int np, int S, double *out, int norm, const double *sc)
 {
     const int n = (int)(blockIdx.x * 4 + threadIdx.x / 32), lane = threadIdx.x & 31;
     if (n >= S) return;
     double s = 0.0;
     for (int k = lane; k < np; k += 32) s += part[(size_t)n * np + k];
     s = warp_sum(s) * WTD_DV;
-    if (lane == 0) out[n] = norm ? 1.0 / sqrt(s) : s;
+    if (lane == 0) out[n] = norm ? 1.0 / sqrt(s) : s * (sc[n] * sc[n]);
 }
 
-/* the ABM update of one chunk of one component of one state.  PASS 0: f_k = h - E y (or read from
- * ring slot NH-1), predictor into y, partial corrector P; 1: corrector into y; 2: norm only;
+/* the ABM update of one chunk of one component of one state, y and h times the state's scale.  PASS 0:
+ * f_k = h - E y (or read from ring slot NH-1), predictor into y, partial corrector P; 1: corrector into y; 2: norm only;
  * 3: f_k only */
 template <typename TY, typename TH, typename TC, int NH, int PASS>
 __global__ void __launch_bounds__(S3::AT) k3s_abm(StepArgs a, const typename cplx<TC>::t *__restrict__ H,
@@ -378,8 +374,8 @@ __global__ void __launch_bounds__(S3::AT) k3s_abm(StepArgs a, const typename cpl
         double2 fk = make_double2(0.0, 0.0), out = y0;
         if (haveH) {
             const double2 h = to_d(hv[k]);
-            fk.x = h.x - E * y0.x;
-            fk.y = h.y - E * y0.y;
+            fk.x = h.x * s - E * y0.x;
+            fk.y = h.y * s - E * y0.y;
         } else if (PASS == 0) {
             fk = to_d(fkg[k]);
         }
@@ -513,14 +509,13 @@ __global__ void __launch_bounds__(S3::LT) k3s_dens_plane(int S, int nchunk, cons
     const double jsgn = comp ? -1.0 : 1.0;
     for (int n = s0; n < s1; n++) {
         const size_t base = ((size_t)comp * S + n) * N + (size_t)x * NYZ;
-        const double f0 = occ[n], w = (comp ? 1.0 - f0 : f0) * wcnt[n], wj = w * jsgn;
-        const TC s = (TC)sc[n];
+        const double f0 = occ[n], w = (comp ? 1.0 - f0 : f0) * wcnt[n] * (sc[n] * sc[n]), wj = w * jsgn;
         if (t == 0 && n + 1 < s1) prefetch_l2(Y + base + N, NYZ * sizeof(TY));
         __syncthreads();
 #pragma unroll 8
         for (int i = t; i < NYZ; i += LT) {
             const TY a = Y[base + i];
-            C z; z.x = a.x * s; z.y = a.y * s;
+            C z; z.x = a.x; z.y = a.y;
             P[(i / NZ) * PITCH + i % NZ] = z;
         }
         __syncthreads();
@@ -592,15 +587,12 @@ __global__ void __launch_bounds__(2 * S3::XL) k3s_dens_x(int S, int nchunk, cons
     const double jsgn = comp ? -1.0 : 1.0;
     for (int n = s0; n < s1; n++) {
         const TC *yr = (const TC *)Y + 2 * (((size_t)comp * S + n) * N + q0 + q) + c;
-        const double f0 = occ[n], w = (comp ? 1.0 - f0 : f0) * wcnt[n], wj = w * jsgn;
-        const TC s = (TC)sc[n];
+        const double f0 = occ[n], w = (comp ? 1.0 - f0 : f0) * wcnt[n] * (sc[n] * sc[n]), wj = w * jsgn;
         if (n + 1 < s1)
             for (int r = lane; r < NX; r += XL) prefetch_l2(Y + ((size_t)comp * S + n + 1) * N + (size_t)r * NYZ + q0, QB * sizeof(TY));
         TC f[NX], l[NX];
 #pragma unroll
         for (int x = 0; x < NX; x++) f[x] = yr[(size_t)2 * x * NYZ];
-#pragma unroll
-        for (int x = 0; x < NX; x++) f[x] *= s;
         circ::line_op<circ::LAP, 0, NX>(f, l);
 #pragma unroll
         for (int x = 0; x < NX; x++) {

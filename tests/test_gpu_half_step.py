@@ -119,3 +119,57 @@ def test_densities_are_those_of_the_returned_states(has_gpu, name, nwf, prec):
         for want, off in (((np.abs(u) ** 2 * f).sum(0), 2), ((np.abs(v) ** 2 * (1.0 - f)).sum(0), 7)):
             assert np.linalg.norm(dens[off * N:(off + 1) * N] - want) < 1e-14 * np.linalg.norm(want)
     r.close()
+
+
+def _h_psi_ragged(proj, psi, pots, params):
+    """H psi of t3d_ragged (3D ASLDA, variable mass, Delta_ext) in numpy: psi [2, S, N], FP64"""
+    n = (proj.nx, proj.ny, proj.nz)
+    N, S = proj.numel, psi.shape[1]
+    c = proj.constants()
+    k, kd = [], []
+    for m, d in zip(n, (proj.dx, proj.dy, proj.dz)):
+        q = np.where(np.arange(m) < m // 2, np.arange(m), np.arange(m) - m) * (2.0 * np.pi / (m * d))
+        k.append(q)
+        kd.append(np.where(np.arange(m) == m // 2, 0.0, q))
+    k2 = k[0][:, None, None] ** 2 + k[1][None, :, None] ** 2 + k[2][None, None, :] ** 2
+    kd = [kd[0][:, None, None], kd[1][None, :, None], kd[2][None, None, :]]
+
+    def spectral(f, mul):
+        g = np.fft.fftn(f.reshape(-1, *n), axes=(1, 2, 3)) * mul
+        return np.fft.ifftn(g, axes=(1, 2, 3)).reshape(f.shape)
+    x = [(np.arange(m) - m // 2) * d for m, d in zip(n, (proj.dx, proj.dy, proj.dz))]
+    L = [m * d for m, d in zip(n, (proj.dx, proj.dy, proj.dz))]
+    dext = params[3] * (1.0 + 0.5j * np.sin(2 * np.pi * x[0] / L[0]))[:, None, None] * np.cos(2 * np.pi * x[1] / L[1])[None, :, None]
+    D = pots[2 * N:4 * N].view(np.complex128) + np.broadcast_to(dext, n).reshape(N)
+    H = np.empty_like(psi)
+    for s in range(2):
+        V, al, A = pots[s * N:(s + 1) * N] - (c["mu_a"], c["mu_b"])[s], pots[(4 + s) * N:(5 + s) * N], pots[(6 + 3 * s) * N:(9 + 3 * s) * N].reshape(3, N)
+        sgn, y, o = (1.0, -1.0)[s], psi[s], psi[1 - s]
+        lap_al = spectral(al[None].astype(complex), -k2)[0].real
+        div = sum(spectral(A[a][None].astype(complex), 1j * kd[a])[0].real for a in range(3))
+        H[s] = sgn * (-0.25 * (al * spectral(y, -k2) + spectral(al * y, -k2)) + (V + 0.25 * lap_al) * y) + (D, D.conj())[s] * o
+        H[s] += -1j * sum(A[a] * spectral(y, 1j * kd[a]) for a in range(3)) - 0.5j * div * y
+    return H
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("prec", [0, 1])
+def test_mixed_h64_forms_h_in_fp64_where_the_line_path_does_not_fit(has_gpu, prec):
+    """f = (H - <H>) psi of the stored states, formed on demand and kept in FP64: on 20 x 18 x 22, which
+    the line path does not take, WTD_MIXED_H64 computes it from the complex64 states in FP64.  Two
+    FP64 evaluations of sums of at most 3 x 22 products per point differ by less than 1e-13 of f;
+    FP32 arithmetic would differ by 1e-7."""
+    from wslda_b200 import TDRun
+    nwf = 7
+    proj, d = inputs("t3d_ragged", nwf)
+    r = TDRun("t3d_ragged", nwf, precision=prec)
+    r.setup(d["states"], d["pots"], d["occ"], d["params"], d["extra"])
+    r.initial_measurement()
+    r.steps(2)
+    f, psi, E = r.history(0).reshape(2, nwf, -1), r.states().reshape(2, nwf, -1), r.qpe()
+    h = _h_psi_ragged(proj, psi, r.potentials(), d["params"])
+    r.close()
+    e = (psi.conj() * h).real.sum(axis=(0, 2)) * proj.dv
+    assert np.abs(E - e).max() < 1e-12 * np.abs(e).max()
+    want = h - e[None, :, None] * psi
+    assert np.linalg.norm(f - want) < 1e-13 * np.linalg.norm(want)

@@ -1272,7 +1272,9 @@ int wtd_create(wtd_ctx **out, int nwf, int precision, int device)
      * =staged the staged path. */
     {
         const char *pp = getenv("WTD_3D_PATH");
-        const bool stream = stream_fits(precision);
+        /* WTD_MIXED_H64 takes it only where the line path, with its FP32 arithmetic, would be the
+         * alternative: elsewhere the staged path forms H of the complex64 states in FP64 */
+        const bool stream = stream_fits(precision) && (precision != WTD_MIXED_H64 || line_fits(precision));
         bool want = stream || precision != WTD_FP64;
         if (pp && strcmp(pp, "line") == 0) want = true;
         if (pp && strcmp(pp, "staged") == 0) want = false;

@@ -173,3 +173,41 @@ def test_mixed_h64_forms_h_in_fp64_where_the_line_path_does_not_fit(has_gpu, pre
     assert np.abs(E - e).max() < 1e-12 * np.abs(e).max()
     want = h - e[None, :, None] * psi
     assert np.linalg.norm(f - want) < 1e-13 * np.linalg.norm(want)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("name,nwf,fail_at", [("t3d_ragged", 9, 1), ("t3d_ragged", 9, 2), ("t2d_slda", 24, 1)])
+def test_failed_density_exchange_leaves_normalised_states(has_gpu, name, nwf, fail_at):
+    """a density exchange that fails inside a block ends the call with an error; the states are left
+    normalised, and the context then runs new states as a fresh one does"""
+    from wslda_b200 import TDRun, WtdError
+    proj, d = inputs(name, nwf)
+    calls = [0]
+
+    def hook(ptr, count, stream):
+        calls[0] += 1
+        if calls[0] > fail_at:
+            raise RuntimeError("exchange refused by the test")
+
+    def fresh(r):
+        r.setup(d["states"], d["pots"], d["occ"], d["params"], d["extra"])
+        r.initial_measurement()
+        r.steps(2)
+        return r.states(), r.densities(), r.potentials()
+    r = TDRun(name, nwf)
+    r.setup(d["states"], d["pots"], d["occ"], d["params"], d["extra"])
+    r.set_density_exchange(hook)
+    r.initial_measurement()
+    with pytest.raises(WtdError):
+        r.steps(3)
+    y = r.states().reshape(2, nwf, -1)
+    norms = (np.abs(y) ** 2).sum(axis=(0, 2)) * proj.dv
+    assert np.abs(norms - 1.0).max() < 1e-12
+    r.set_density_exchange(None)
+    got = fresh(r)
+    r.close()
+    other = TDRun(name, nwf)
+    want = fresh(other)
+    other.close()
+    for a, b in zip(got, want):
+        assert np.array_equal(a, b)

@@ -845,6 +845,20 @@ static int stream_step(wtd_ctx *c, bool last)
     return WTD_OK;
 }
 
+/* nsteps steps; where one fails (the exchange of the densities) the states are left normalised, as on
+ * the other paths, and their scales 1 */
+static int stream_steps(wtd_ctx *c, int nsteps)
+{
+    for (int s = 0; s < nsteps; s++) {
+        const int r = stream_step(c, s == nsteps - 1);
+        if (r != WTD_OK) {
+            stream_form(c, [&](auto f) { return decltype(f)::rescale(c); });
+            return r;
+        }
+    }
+    return WTD_OK;
+}
+
 static int stream_initial(wtd_ctx *c)
 {
     WTD_TRY(stream_pass(c, 2, true, true));
@@ -861,7 +875,7 @@ static int stream_coef_var(wtd_ctx *) { return WTD_ERR_UNSUPPORTED; }
 static size_t stream_slot_words(const wtd_ctx *) { return 0; }
 static size_t stream_part_words(const wtd_ctx *) { return 0; }
 static int stream_pass(wtd_ctx *, int, bool, bool) { return WTD_ERR_UNSUPPORTED; }
-static int stream_step(wtd_ctx *, bool) { return WTD_ERR_UNSUPPORTED; }
+static int stream_steps(wtd_ctx *, int) { return WTD_ERR_UNSUPPORTED; }
 static int stream_initial(wtd_ctx *) { return WTD_ERR_UNSUPPORTED; }
 static int stream_setup(wtd_ctx *, int) { return WTD_ERR_UNSUPPORTED; }
 static int stream_subset(wtd_ctx *, const double *, double *) { return WTD_ERR_UNSUPPORTED; }
@@ -1604,10 +1618,7 @@ int wtd_steps(wtd_ctx *c, int nsteps)
         for (int s = 0; s < nsteps; s++) WTD_TRY(staged_step(c, s == nsteps - 1));
         return WTD_OK;
     }
-    if (c->stream) {
-        for (int s = 0; s < nsteps; s++) WTD_TRY(stream_step(c, s == nsteps - 1));
-        return WTD_OK;
-    }
+    if (c->stream) return stream_steps(c, nsteps);
     if (c->line) {
         for (int s = 0; s < nsteps; s++) WTD_TRY(line_step(c, s == nsteps - 1));
         return WTD_OK;

@@ -60,9 +60,13 @@ def test_variable_mass_many_states(has_gpu, name):
                                                 ("c5_slda3d", 4, 1, 1e-5), ("c5_slda3d", 4, 2, 1e-5), ("t2d_big", 8, 1, 1e-6)])
 def test_mixed_forms_track_fp64(has_gpu, name, nwf, prec, tol):
     """the FP32-mixed forms (complex64 states; FP64 or complex64 history) against the FP64
-    oracle over a measurement block: the fused lattices and the 3D line path (c3_aslda3d,
-    c5_slda3d) compute the transforms and H psi in FP32; the 2D plane/pencil lattice (t2d_big)
+    oracle over a measurement block: the fused lattices and the 3D stream path (c3_aslda3d,
+    c5_slda3d) compute the derivatives and H psi in FP32; the 2D plane/pencil lattice (t2d_big)
     keeps FP64 arithmetic and rounds the states to complex64 after each renormalisation"""
+    _track_fp64(name, nwf, prec, tol)
+
+
+def _track_fp64(name, nwf, prec, tol):
     o = run_oracle(name, nwf, 3, 1)
     g = run_gpu(name, nwf, 3, 1, precision=prec)
     n = o["densities"].size // 12
@@ -71,6 +75,40 @@ def test_mixed_forms_track_fp64(has_gpu, name, nwf, prec, tol):
         assert errs[k] < tol, (name, prec, k, errs[k])
     e_o, e_g = o["energy"][:7].sum(), g["energy"][:7].sum()
     assert abs(e_g - e_o) / abs(e_o) < tol
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("name,nwf,prec", [("c3_aslda3d", 8, 1), ("c3_aslda3d", 8, 2), ("c5_slda3d", 4, 2), ("t3d_long", 7, 1),
+                                           ("t3d_long", 7, 2)])
+def test_line_path_mixed_forms(has_gpu, monkeypatch, name, nwf, prec):
+    """the FP32-mixed forms on the 3D line path, asked for on 32^3 and 48^3 and the default on 72 x 16
+    x 16, to FP32 rounding as test_mixed_forms_track_fp64"""
+    if name != "t3d_long":
+        monkeypatch.setenv("WTD_3D_PATH", "line")
+    _track_fp64(name, nwf, prec, 1e-5)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("path", ["staged", "line"])
+def test_t3d_long_axis_beyond_64(has_gpu, monkeypatch, path):
+    """3D ASLDA 72 x 16 x 16: an axis beyond the stream path's 64 points, in FP64 on the staged path (the
+    default) and the line path"""
+    monkeypatch.setenv("WTD_3D_PATH", path)
+    _compare("t3d_long", nwf=7, nsteps=3, nmeas=2)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("nwf", [2, 5])
+def test_t3d_wide_axes_to_64(has_gpu, nwf):
+    """the stream path at the upper end of its range, with unequal axes and constant mass (50 x 54 x 64,
+    SLDA), from two states on"""
+    _compare("t3d_wide", nwf=nwf, nsteps=2, nmeas=1)
+
+
+@pytest.mark.gpu
+def test_t3d_wide_h32(has_gpu):
+    """the same lattice in the all-FP32 form"""
+    _track_fp64("t3d_wide", 4, 2, 1e-5)
 
 
 @pytest.mark.gpu
@@ -124,18 +162,18 @@ def test_c4_bdg2d_small_s(has_gpu):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("path", ["staged", "line"])
+@pytest.mark.parametrize("path", ["staged", "line", "stream"])
 def test_c3_aslda3d_small_s(has_gpu, monkeypatch, path):
-    """3D ASLDA 32^3 (state larger than one CTA) in FP64: the staged plane/pencil path (the FP64
-    default) and the 3D line path (the FP32 forms' path)"""
+    """3D ASLDA 32^3 (state larger than one CTA) in FP64 on the staged plane/pencil path, the line
+    path and the stream path (the default)"""
     monkeypatch.setenv("WTD_3D_PATH", path)
     _compare("c3_aslda3d", nwf=8, nsteps=2, nmeas=1)
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("path", ["staged", "line"])
+@pytest.mark.parametrize("path", ["staged", "line", "stream"])
 def test_c5_slda3d_small_s(has_gpu, monkeypatch, path):
-    """3D SLDA 48^3 (radix-3 axes) in FP64 on both 3D paths."""
+    """3D SLDA 48^3 (radix-3 axes) in FP64 on the three 3D paths."""
     monkeypatch.setenv("WTD_3D_PATH", path)
     _compare("c5_slda3d", nwf=4, nsteps=2, nmeas=1)
 
@@ -166,7 +204,7 @@ def test_t3d_ragged_mixed_forms(has_gpu, nwf, prec):
 def test_high_k_filters(has_gpu, name, nwf, nsteps, mode):
     """runs with the high-k filters on: mode 1 filters the effective masses after every
     functional evaluation (pca.c:1448-1453), mode 2 the pairing field too; fused path (t1d,
-    t2d, t3d) and staged plane/pencil path (c3, 32^3)"""
+    t2d, t3d) and 3D stream path (c3, 32^3)"""
     import sys, os
     sys.path.insert(0, os.path.dirname(os.path.abspath(__file__)))
     from golden.make_golden import hkf_params
@@ -187,6 +225,10 @@ def test_t2d_big_staged(has_gpu):
 def test_selfstart(has_gpu, name, nwf, nsteps, nmeas):
     """Taylor self-start of the history (pca.c:1086-1330) then the ABM steps: constant and
     variable mass, 1D/2D/3D, fused and plane/pencil lattices"""
+    _selfstart(name, nwf, nsteps, nmeas)
+
+
+def _selfstart(name, nwf, nsteps, nmeas):
     o = run_oracle(name, nwf, nsteps, nmeas, selfstart=True)
     g = run_gpu(name, nwf, nsteps, nmeas, selfstart=True)
     n = o["densities"].size // 12
@@ -206,6 +248,10 @@ def test_quantum_friction(has_gpu, name, nwf, nsteps, nmeas):
     """steps with quantum friction switched on over the run (ramp included): friction
     densities, particle control and the friction-modified H (pca_kernels.cu:497-539), on the
     fused lattices and on the plane/pencil path (c3_aslda3d, t2d_big)"""
+    _friction(name, nwf, nsteps, nmeas)
+
+
+def _friction(name, nwf, nsteps, nmeas):
     import sys, os
     sys.path.insert(0, os.path.dirname(os.path.abspath(__file__)))
     from golden.make_golden import QF_PARAMS
@@ -225,6 +271,24 @@ def test_quantum_friction(has_gpu, name, nwf, nsteps, nmeas):
 def test_subset_densities(has_gpu, name, nwf):
     """densities of a weighted subset of the states after a few steps (subset tracking,
     pca.c:1056-1066) against the oracle's calculate_densities with the same weights"""
+    _subset(name, nwf)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("what", ["friction", "selfstart", "subset"])
+def test_line_path_other_calls(has_gpu, monkeypatch, what):
+    """quantum friction (which continues on the staged path), self-start and subset densities of a
+    context on the 3D line path"""
+    monkeypatch.setenv("WTD_3D_PATH", "line")
+    if what == "friction":
+        _friction("c3_aslda3d", 8, 2, 1)
+    elif what == "selfstart":
+        _selfstart("c3_aslda3d", 8, 2, 1)
+    else:
+        _subset("c3_aslda3d", 8)
+
+
+def _subset(name, nwf):
     from oracle_lib import Oracle
     from wslda_b200 import TDRun
     from parity_util import inputs

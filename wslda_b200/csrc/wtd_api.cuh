@@ -1205,6 +1205,26 @@ static int occupancy_t(int block)
     }
 }
 
+/* the path of a context of the given precision form.  On lattices beyond one CTA:
+ *   the stream path where it fits (StreamFit: 3D, axes of at most 64 points whose planes fit shared
+ *   memory), but WTD_MIXED_H64 only where the line path fits too: both compute in FP32, and without
+ *   the line path the staged path forms H of the complex64 states in FP64;
+ *   else the line path (LineCfg: elongated 3D lattices) for the FP32-mixed forms;
+ *   else the staged path, which WTD_MIXED_H32 does not have.
+ * WTD_3D_PATH=stream, line or staged asks for one of them, and takes it where it fits. */
+enum { PATH_FUSED, PATH_STAGED, PATH_LINE, PATH_STREAM };
+static int path_of(int precision)
+{
+    if (!WTD_BIG) return PATH_FUSED;
+    const char *ask = getenv("WTD_3D_PATH");
+    const bool line = line_fits(precision), stream = stream_fits(precision);
+    if (ask && strcmp(ask, "staged") == 0) return PATH_STAGED;
+    if (ask && strcmp(ask, "line") == 0 && line) return PATH_LINE;
+    if (ask && strcmp(ask, "stream") == 0 && stream) return PATH_STREAM;
+    if (stream && (precision != WTD_MIXED_H64 || line)) return PATH_STREAM;
+    return line && precision != WTD_FP64 ? PATH_LINE : PATH_STAGED;
+}
+
 static int occupancy_per_sm(wtd_ctx *c)
 {
     if (c->prec == WTD_FP64) return occupancy_t<double2, double2, double>(c->block);
@@ -1280,22 +1300,10 @@ int wtd_create(wtd_ctx **out, int nwf, int precision, int device)
         const char *pf = getenv("WTD_PREFETCH");
         if (pf) c->prefetch = atoi(pf) & 15;
     }
-    /* lattices beyond one CTA.  Where it fits (3D, axes of at most 64 points) every form takes the
-     * stream path; elsewhere the FP32-mixed forms take the 3D line path and FP64 the staged path,
-     * each the faster there.  WTD_3D_PATH=line selects the stream (or line) path for every form,
-     * =staged the staged path. */
-    {
-        const char *pp = getenv("WTD_3D_PATH");
-        /* WTD_MIXED_H64 takes it only where the line path, with its FP32 arithmetic, would be the
-         * alternative: elsewhere the staged path forms H of the complex64 states in FP64 */
-        const bool stream = stream_fits(precision) && (precision != WTD_MIXED_H64 || line_fits(precision));
-        bool want = stream || precision != WTD_FP64;
-        if (pp && strcmp(pp, "line") == 0) want = true;
-        if (pp && strcmp(pp, "staged") == 0) want = false;
-        c->stream = (stream && want) ? 1 : 0;
-        c->line = (!c->stream && WTD_BIG && line_fits(precision) && want) ? 1 : 0;
-    }
-    c->staged = (WTD_BIG && !c->line && !c->stream) ? 1 : 0;
+    const int path = path_of(precision);
+    c->stream = path == PATH_STREAM;
+    c->line = path == PATH_LINE;
+    c->staged = path == PATH_STAGED;
     if (c->staged && precision == WTD_MIXED_H32) { free(c); return WTD_ERR_UNSUPPORTED; }
     if (c->line && line_setup(c, nsm) != WTD_OK) { free(c); return WTD_ERR_CUDA; }
     if (c->stream && stream_setup(c, nsm) != WTD_OK) { free(c); return WTD_ERR_CUDA; }

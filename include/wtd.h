@@ -60,7 +60,8 @@ typedef struct wtd_ctx wtd_ctx;
 /* lattice and build facts of this library: dims[3], numel, codedim, scheme history length,
  * functional id (111 SLDA, 112 ASLDA, 113 BDG, 114 CUSTOMEDF), const-mass flag */
 int wtd_info(int *dims, int *numel, int *codedim, int *nhist, int *functional, int *const_mass);
-/* device bytes a context of nwf states in the given precision needs */
+/* device bytes a context of nwf states in the given precision needs, on the path that wtd_create would
+ * take; the adjoint's, the self-start's and the subset densities' work arrays come on top */
 size_t wtd_device_bytes(int nwf, int precision);
 
 int wtd_create(wtd_ctx **ctx, int nwf, int precision, int device);

@@ -211,3 +211,29 @@ def test_failed_density_exchange_leaves_normalised_states(has_gpu, name, nwf, fa
     other.close()
     for a, b in zip(got, want):
         assert np.array_equal(a, b)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("name,nwf,prec,path", [("c3_aslda3d", 400, 0, None), ("c3_aslda3d", 400, 1, None), ("c3_aslda3d", 400, 2, None),
+                                                ("c3_aslda3d", 400, 0, "staged"), ("c3_aslda3d", 400, 2, "line"),
+                                                ("t3d_ragged", 1500, 1, None), ("t2d_big", 600, 0, None), ("t2d_big", 600, 1, None),
+                                                ("c2_slda2d", 3000, 0, None)])
+def test_device_bytes_are_those_of_the_path(has_gpu, monkeypatch, name, nwf, prec, path):
+    """wtd_device_bytes against the device memory that a context takes, on every path.  It leaves out
+    nothing that grows with the states, so the two differ by the rounding of two dozen allocations
+    (2 MiB each) and by the estimate of the density slots (300 CTAs; the paths take between 148 and
+    600 of 12 to 16 words a point): 600 x 16 x N doubles."""
+    import torch
+    from wslda_b200 import TDRun
+    if path:
+        monkeypatch.setenv("WTD_3D_PATH", path)
+    TDRun(name, 1, precision=prec).close()          # modules loaded, context created
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    r = TDRun(name, nwf, precision=prec)
+    used = free - torch.cuda.mem_get_info()[0]
+    N = r.N
+    want = r.lib.wtd_device_bytes(nwf, prec)
+    r.close()
+    assert abs(used - want) < 24 * 2 ** 21 + 300 * 16 * N * 8, (used, want)
+    assert abs(used - want) < 0.1 * used, (used, want)

@@ -784,7 +784,7 @@ template <class F> static int stream_form(wtd_ctx *c, F f)
     return WTD_ERR_UNSUPPORTED;
 }
 static size_t stream_slot_words(const wtd_ctx *c) { return (size_t)(4 * c->gpt + 6 * c->gpl + 4 * c->gx) * S3::N; }
-static size_t stream_part_words(const wtd_ctx *c) { return (size_t)c->S * 2 * (S3::NQB > S3::ACH ? S3::NQB : S3::ACH); }
+static size_t stream_part_words(int S) { return (size_t)S * 2 * (S3::NQB > S3::ACH ? S3::NQB : S3::ACH); }
 
 /* one half step's kernels (pass 0: H y_k + predictor, 1: H y_pred + corrector, 2: norms and
  * densities, 3: f_k only), timed like the fused passes when timing is on */
@@ -873,7 +873,7 @@ static int stream_setup(wtd_ctx *c, int nsm)
 static bool stream_fits(int) { return false; }
 static int stream_coef_var(wtd_ctx *) { return WTD_ERR_UNSUPPORTED; }
 static size_t stream_slot_words(const wtd_ctx *) { return 0; }
-static size_t stream_part_words(const wtd_ctx *) { return 0; }
+static size_t stream_part_words(int) { return 0; }
 static int stream_pass(wtd_ctx *, int, bool, bool) { return WTD_ERR_UNSUPPORTED; }
 static int stream_steps(wtd_ctx *, int) { return WTD_ERR_UNSUPPORTED; }
 static int stream_initial(wtd_ctx *) { return WTD_ERR_UNSUPPORTED; }
@@ -1250,10 +1250,21 @@ int wtd_info(int *dims, int *numel, int *codedim, int *nhist, int *functional, i
 
 size_t wtd_device_bytes(int nwf, int precision)
 {
-    size_t n2 = (size_t)2 * nwf * WTD_NUMEL;
-    size_t b = n2 * (elem_bytes_y(precision) + WTD_NHIST * elem_bytes_h(precision)) +
-               (size_t)300 * 16 * WTD_NUMEL * sizeof(double);
-    if (WTD_BIG) b += n2 * sizeof(double2) * ((CODEDIM >= 3 ? 4 : 3) + (WTD_VAR ? 1 : 0));
+    if (nwf <= 0 || precision < 0 || precision > 2) return 0;
+    const size_t N = WTD_NUMEL, S = (size_t)nwf, n2 = 2 * S * N;
+    const int path = path_of(precision);
+    /* states, ring, O(N) arrays (coefficients, densities, potentials, friction, energies) and the density
+     * slots of 300 CTAs (two per SM) */
+    size_t b = n2 * (elem_bytes_y(precision) + WTD_NHIST * elem_bytes_h(precision)) + 4 * S * sizeof(double) +
+               (CF_COUNT + 16 + 4 + 12 + TDWSLDAITEMS + (S < 300 ? S : 300) * 16) * N * sizeof(double);
+    if (precision != WTD_FP64) b += WTD_XFER * sizeof(double2);
+    if (path != PATH_FUSED) b += 2 * N * sizeof(double2);
+    if (path == PATH_STAGED) {
+        b += n2 * sizeof(double2) * ((CODEDIM >= 3 ? 4 : 3) + (WTD_VAR ? 1 : 0));
+        if (precision != WTD_FP64) b += n2 * sizeof(double2);
+    } else if (path != PATH_FUSED)
+        b += n2 * (precision == WTD_FP64 ? sizeof(double2) : sizeof(float2));
+    if (path == PATH_STREAM) b += (S + stream_part_words(nwf)) * sizeof(double);
     return b;
 }
 
@@ -1346,7 +1357,7 @@ int wtd_create(wtd_ctx **out, int nwf, int precision, int device)
     }
     if (c->stream) {
         ALLOC(c->sc, nwf * sizeof(double));
-        ALLOC(c->part, stream_part_words(c) * sizeof(double));
+        ALLOC(c->part, stream_part_words(nwf) * sizeof(double));
     }
     if (c->staged) {
         ALLOC(c->ddx, n2 * sizeof(double2));

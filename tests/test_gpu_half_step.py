@@ -237,3 +237,30 @@ def test_device_bytes_are_those_of_the_path(has_gpu, monkeypatch, name, nwf, pre
     r.close()
     assert abs(used - want) < 24 * 2 ** 21 + 300 * 16 * N * 8, (used, want)
     assert abs(used - want) < 0.1 * used, (used, want)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("name,nwf", [("t3d_ragged", 9), ("t2d_slda", 24)])
+def test_subset_densities_report_a_failed_wait(has_gpu, name, nwf):
+    """the error of the call's last wait is returned and not dropped.  The wait is made to fail on the
+    host, without a fault: a stream in capture refuses to be waited for, and nothing of what was
+    queued runs; the context is used on afterwards"""
+    from wslda_b200 import TDRun, WtdError
+    import torch  # noqa: F401  (its CUDA runtime is the one loaded here)
+    rt = ctypes.CDLL("libcudart.so.12")
+    proj, d = inputs(name, nwf)
+    r = TDRun(name, nwf)
+    r.setup(d["states"], d["pots"], d["occ"], d["params"], d["extra"])
+    r.initial_measurement()
+    w = np.ones(nwf)
+    want = r.subset_densities(w)
+    st, graph = ctypes.c_void_p(r.stream()), ctypes.c_void_p()
+    assert rt.cudaStreamBeginCapture(st, 2) == 0          # relaxed: allocations stay allowed
+    try:
+        with pytest.raises(WtdError):
+            r.subset_densities(w)
+    finally:
+        rt.cudaStreamEndCapture(st, ctypes.byref(graph))   # the refused wait has ended the capture
+        rt.cudaGetLastError()
+    assert np.array_equal(r.subset_densities(w), want)
+    r.close()

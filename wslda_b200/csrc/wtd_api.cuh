@@ -1823,6 +1823,15 @@ int wtd_set_density_exchange(wtd_ctx *c, wtd_exchange_fn fn, void *user)
 
 } /* extern "C" */
 
+/* waits for the context's stream before work arrays are freed; an error is returned, and cleared so that
+ * the next call's launches do not report it again */
+static int wait_stream(wtd_ctx *c)
+{
+    const int e = wtd_cuerr(cudaStreamSynchronize(c->st));
+    if (e != WTD_OK) cudaGetLastError();
+    return e;
+}
+
 /* ---------------------------------------------------------------------------------------
  * Taylor self-start of the ABM history (pca.c:1086-1330, input selfstart 1), FP64: the q
  * first steps are taken with exp(-i H dt) expanded to exp_iters orders (midpoint potentials
@@ -2006,8 +2015,9 @@ extern "C" int wtd_selfstart(wtd_ctx *c)
     if (!r) r = get(&w.rec, (size_t)WTD_NHIST * NS);
     if (!r) r = get((double2 **)&w.qs, (size_t)c->S);
     if (!r) r = selfstart_run(c, w);
-    cudaStreamSynchronize(c->st);
+    const int e = wait_stream(c);
     for (void *q : w.own) cudaFree(q);
+    if (!r) r = e;
     return r ? r : wtd_cuerr(cudaGetLastError());
 }
 
@@ -2044,9 +2054,9 @@ extern "C" int wtd_subset_densities(wtd_ctx *c, const double *weights, double *h
     if (!r && c->stream) {
         r = stream_subset(c, dw, out);
         if (!r) r = wtd_cuerr(cudaMemcpyAsync(host12, out, 12 * N * sizeof(double), cudaMemcpyDeviceToHost, c->st));
-        cudaStreamSynchronize(c->st);
+        const int e = wait_stream(c);
         for (void *q : w.own) cudaFree(q);
-        return r;
+        return r ? r : e;
     }
     if (!r) r = ss_derivs(c, w, (const double2 *)c->y, 1);
     if (!r) {
@@ -2069,9 +2079,9 @@ extern "C" int wtd_subset_densities(wtd_ctx *c, const double *weights, double *h
         }
     }
     if (!r) r = wtd_cuerr(cudaMemcpyAsync(host12, out, 12 * N * sizeof(double), cudaMemcpyDeviceToHost, c->st));
-    cudaStreamSynchronize(c->st);
+    const int e = wait_stream(c);
     for (void *q : w.own) cudaFree(q);
-    return r;
+    return r ? r : e;
 }
 
 /* ---------------------------------------------------------------------------------------

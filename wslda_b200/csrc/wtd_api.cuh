@@ -550,13 +550,14 @@ static int staged_potentials(wtd_ctx *c, int it)
     return WTD_OK;
 }
 
-/* threads of the kernels with one CTA per state: more where the states are too few to fill the GPU
- * with CTAs of 256 */
-static int staged_threads(const wtd_ctx *c) { return c->S < 4 * 148 && WTD_NUMEL >= 4096 ? 512 : 256; }
+/* threads of the kernels with one CTA per state.  Lattices beyond one CTA have at least 6,000 points; 512
+ * threads against 256, ms per step of 160x96 in FP64: 40 states 0.96 / 1.19, 148 1.88 / 2.16, 301 3.36
+ * / 3.36, 700 6.74 / 6.95, 1500 13.61 / 13.65; of 20x18x22: 40 states 1.71 / 1.80, 300 8.89 / 8.87 */
+static constexpr int STAGED_THREADS = 512;
 
 static int staged_hamiltonian(wtd_ctx *c, double2 *out)
 {
-    k_hamiltonian_compat<<<c->S, staged_threads(c), 0, c->st>>>(c->S, st_y(c), out, c->ddx, c->ddy, c->ddz, c->dlap,
+    k_hamiltonian_compat<<<c->S, STAGED_THREADS, 0, c->st>>>(c->S, st_y(c), out, c->ddx, c->ddy, c->ddz, c->dlap,
                                                   c->dalap, c->cf, c->kp2, c->qpe, NULL);
     WTD_LAUNCHED(c);
     return WTD_OK;
@@ -565,7 +566,7 @@ static int staged_hamiltonian(wtd_ctx *c, double2 *out)
 static int staged_initial(wtd_ctx *c)
 {
     WTD_TRY(st_load(c));
-    k_normalize<<<c->S, staged_threads(c), 0, c->st>>>(c->S, st_y(c));
+    k_normalize<<<c->S, STAGED_THREADS, 0, c->st>>>(c->S, st_y(c));
     WTD_LAUNCHED(c);
     WTD_TRY(st_round(c));
     WTD_TRY(staged_derivs(c, true));
@@ -593,7 +594,7 @@ static int staged_step(wtd_ctx *c, bool last)
     else if (NH == 4) k_abm_step1<4><<<nb, 256, 0, c->st>>>(M, Y, f[0], f[1], f[2], f[3], NULL, c->dt);
     else k_abm_step1<5><<<nb, 256, 0, c->st>>>(M, Y, f[0], f[1], f[2], f[3], f[4], c->dt);
     WTD_LAUNCHED(c);
-    k_normalize<<<c->S, staged_threads(c), 0, c->st>>>(c->S, Y);
+    k_normalize<<<c->S, STAGED_THREADS, 0, c->st>>>(c->S, Y);
     WTD_LAUNCHED(c);
     WTD_TRY(st_round(c));
     WTD_TRY(staged_derivs(c, var || qf));
@@ -604,7 +605,7 @@ static int staged_step(wtd_ctx *c, bool last)
     const double cc = (NH == 3) ? 9. / 24. : 251. / 720.;
     k_abm_step4<<<nb, 256, 0, c->st>>>(M, c->dlap, Y, f[NH - 1], c->dt, cc);
     WTD_LAUNCHED(c);
-    k_normalize<<<c->S, staged_threads(c), 0, c->st>>>(c->S, Y);
+    k_normalize<<<c->S, STAGED_THREADS, 0, c->st>>>(c->S, Y);
     WTD_LAUNCHED(c);
     WTD_TRY(st_round(c));
     const bool g = var || last || qf;

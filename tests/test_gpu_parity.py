@@ -220,6 +220,14 @@ def test_t2d_big_staged(has_gpu):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("nwf", [9, 13])
+def test_t2d_ragged_rows(has_gpu, nwf):
+    """2D 90x84 ASLDA beyond one CTA: 1620 or 2340 rows of all fields, which the groups of 16 rows of a CTA
+    do not divide, and a group that spans two fields"""
+    _compare("t2d_ragged", nwf=nwf, nsteps=3, nmeas=1)
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("name,nwf,nsteps,nmeas", [("t2d_slda", 24, 3, 2), ("t1d_aslda", 24, 3, 2), ("c4_bdg2d", 16, 4, 1),
                                                    ("c3_aslda3d", 8, 2, 1), ("t2d_vext", 24, 3, 1)])
 def test_selfstart(has_gpu, name, nwf, nsteps, nmeas):

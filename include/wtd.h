@@ -44,8 +44,9 @@ typedef struct wtd_ctx wtd_ctx;
 
 /* precision forms */
 #define WTD_FP64 0        /* states, history, FFT and H psi in FP64 (drop-in form) */
-#define WTD_MIXED_H64 1   /* states, FFT and H psi in FP32; ABM history/P stored in FP64 */
-#define WTD_MIXED_H32 2   /* states, history, FFT and H psi in FP32; ABM sums, norms, densities FP64 */
+#define WTD_MIXED_H64 1   /* states, derivatives and H psi in FP32; ABM history/P stored in FP64 (on the
+                           * staged path, large 2D and some 3D lattices, H of the FP32 states in FP64) */
+#define WTD_MIXED_H32 2   /* states, history, derivatives and H psi in FP32; ABM sums, norms, densities FP64 */
 
 /* error codes */
 #define WTD_OK 0
@@ -201,7 +202,9 @@ int wtd_set_high_k_filter(wtd_ctx *ctx, int mode, double mu, double T);
  * (pca_utils.c:779-790, 1055-1060) is on, the friction densities are accumulated with the
  * gradient densities and H is built from V_s - U_s alpha/nF and the phase and particle-control
  * corrections of delta (pca_kernels.cu:497-539); the potentials themselves are not changed.
- * All coefficients 0 turns it off.  Fused-path lattices only (WTD_ERR_UNSUPPORTED otherwise). */
+ * All coefficients 0 turns it off.  On 3D lattices beyond one CTA the run continues on the staged
+ * path, in FP64 only (WTD_ERR_UNSUPPORTED in the mixed forms there; WTD_ERR_NOMEM where its
+ * derivative arrays do not fit). */
 int wtd_set_quantum_friction(wtd_ctx *ctx, double qfalpha, double qfbeta, double qfgamma, double qfNreq,
                              double qfstart, double qfstop, double qfswitch);
 

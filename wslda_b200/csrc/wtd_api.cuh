@@ -52,7 +52,7 @@ struct wtd_ctx {
     int ncl;                    /* clusters of the x-line kernel */
     int g2;                     /* state chunks of the plane density kernel */
     int p1grid;                 /* CTAs of the plane H kernel */
-    /* stream path (wtd_stream3d.cuh), the form of the line path on axes of at most 64 points */
+    /* stream path (wtd_stream3d.cuh) */
     int stream;
     double *sc, *part;          /* scale 1/norm of every state; partial sums of <H> and the norm */
     int xgrid;                  /* CTAs of the x kernel */
@@ -321,8 +321,7 @@ static int coef_var(wtd_ctx *c)
     return WTD_OK;
 }
 
-/* per-point H coefficients from the potentials at time index it (variable
- mass: lap alpha /4
+/* per-point H coefficients from the potentials at time index it (variable mass: lap alpha /4
  * and -div A /2 by spectral derivatives) */
 static int coef_from_pots(wtd_ctx *c, int it, const double *fld = NULL)
 {
@@ -534,13 +533,9 @@ static int staged_derivs(wtd_ctx *c, bool grads)
 
 static int staged_potentials(wtd_ctx *c, int it)
 {
-    constexpr int N = WTD_NUMEL;
-    wslda_density D = convert_into_wslda_density(c->dens, N);
-    wslda_potential P = convert_into_wslda_potential(c->pots, N, NULL);
-    int pb = (N + 127) / 128;
-    (void)D; (void)pb;
     WTD_TRY(functional_coef(c, it));
 #ifndef FAST_CONST_EFFECTIVE_MASS_MODE
+    wslda_potential P = convert_into_wslda_potential(c->pots, WTD_NUMEL, NULL);
     /* lap(alpha psi) for the variable-mass kinetic term (pca.c:1455-1456), the product with
      * alpha taken as the fields are loaded */
     WTD_TRY(big_derivs_sep(st_y(c), 2 * c->S, c->dalap, NULL, NULL, NULL, P.alpha_a, P.alpha_b, c->tw, c->ktab, c->st));
@@ -621,7 +616,8 @@ static int staged_step(wtd_ctx *c, bool last)
 }
 
 /* ---------------------------------------------------------------------------------------
- * stream path (3D lattices beyond one CTA with axes of at most 64 points, wtd_stream3d.cuh)
+ * stream path (3D lattices beyond one CTA with axes of at most 64 points, where StreamFit holds:
+ * wtd_stream3d.cuh)
  * -------------------------------------------------------------------------------------*/
 #if CODEDIM == 3
 template <typename TC> struct StreamFit {
@@ -1208,10 +1204,16 @@ static int occupancy_t(int block)
 
 /* the path of a context of the given precision form.  On lattices beyond one CTA:
  *   the stream path where it fits (StreamFit: 3D, axes of at most 64 points whose planes fit shared
- *   memory), but WTD_MIXED_H64 only where the line path fits too: both compute in FP32, and without
- *   the line path the staged path forms H of the complex64 states in FP64;
- *   else the line path (LineCfg: elongated 3D lattices) for the FP32-mixed forms;
- *   else the staged path, which WTD_MIXED_H32 does not have.
+ *   memory; figures in wtd_stream3d.cuh), but WTD_MIXED_H64 only where the line path fits too: both
+ *   compute in FP32, and without the line path the staged path forms H of the complex64 states in
+ *   FP64;
+ *   else the line path for the FP32-mixed forms.  LineCfg holds for 32^3, 48^3 and elongated lattices
+ *   (72x16x16, 128x32x32), not for 64^3 or 80x64x64.  It is the only path of WTD_MIXED_H32 there.
+ *   WTD_MIXED_H64 takes half the memory of the staged path on it (one FP32 array of h against five or
+ *   six FP64 arrays), but is the slower: 72x16x16 1000 states 83 ms per step against 14, 128x32x32
+ *   400 states 118 against 40, 32x32x128 81 against 43;
+ *   else the staged path, which WTD_MIXED_H32 does not have.  FP64 is faster on it than on the line
+ *   path (72x16x16 1000 states 13.7 ms per step against 88).
  * WTD_3D_PATH=stream, line or staged asks for one of them, and takes it where it fits. */
 enum { PATH_FUSED, PATH_STAGED, PATH_LINE, PATH_STREAM };
 static int path_of(int precision)
@@ -1333,7 +1335,8 @@ int wtd_create(wtd_ctx **out, int nwf, int precision, int device)
     ALLOC(c->wcnt, nwf * sizeof(double));
     {
         /* density slots: per CTA of the fused passes (12 N words, 16 N with quantum friction);
-         * on the line path per cluster and per plane chunk (12 N words) */
+         * on the line path per cluster and per plane chunk (12 N words), on the stream path per chunk
+         * of states (stream_slot_words) */
         size_t slots = (size_t)c->grid * 16 * N;
         if (c->line && (size_t)(c->ncl + c->g2) * 12 * N > slots) slots = (size_t)(c->ncl + c->g2) * 12 * N;
         if (c->stream && stream_slot_words(c) > slots) slots = stream_slot_words(c);

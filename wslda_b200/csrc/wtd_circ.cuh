@@ -12,11 +12,11 @@
  *     f_{j+n/2}) and a skew-circulant, antiperiodic, of n/2 (m_j = f_j - f_{j+n/2}), within each
  *     half; recursively on p while n is even.
  *
- * For n = 32 the laplacian costs 178 multiply-adds and about 110 additions of a real line, with
+ * For n = 32 the laplacian costs 174 multiply-adds and 164 additions of a real line, with
  * coefficients that are compile-time constants; the forward and inverse transforms it replaces
  * cost about 700 operations of a complex line each, with twiddle loads, exchanges between the
  * threads of a line and barriers.  Rounding is that of sums of n products with
- * sum |t| <= (2/3) max |k^2|.
+ * sum_d |t(d)| = max k^2.
  */
 #ifndef WTD_CIRC_CUH
 #define WTD_CIRC_CUH

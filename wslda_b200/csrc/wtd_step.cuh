@@ -149,8 +149,9 @@ __device__ __forceinline__ void kmul(C *buf, const double (*kt)[WTD_KT])
 template <class G, typename TC, bool VAR> struct FusedCfg {
     typedef CircGeo<G> CG;
     /* FP64 lines of more than 48 points need 255 registers, which leaves 256 threads an SM: the
-     * laplacian is faster all the same (64^2: 4.6 us a field against 6.6 us) but pass A's streaming
-     * phases, which live on loads in flight, lose more (8192 states: 2.74 ms against 2.15 ms) */
+     * laplacian is faster all the same (64^2: 4.6 us a field against 6.6 us) but the streaming phases,
+     * which live on loads in flight, lose more, in every pass (64^2, 8192 states, lines / transforms:
+     * pass A 2.77 / 2.14 ms, pass B 1.69 / 1.57 ms without gradients and 8.80 / 4.31 ms with them) */
     static constexpr bool circ = CG::fits && (sizeof(TC) == 4 || CG::nmax <= 48);
     typedef typename std::conditional<circ, CG, G>::type Lay;   /* layout of a field in shared memory */
     /* threads.  Lines of more than 32 points take 128 to 255 registers in FP64, so such lattices
@@ -159,9 +160,10 @@ template <class G, typename TC, bool VAR> struct FusedCfg {
     static constexpr int lines = (CG::total + 31) / 32 * 32;
     static constexpr int pts = (G::ntot + 31) / 32 * 32;
     /* 3D with constant mass: a component has more lines than the block has threads, and they are
-     * read from global memory (L2, L1) in rounds instead of from a staged copy: pass A of 895 states
-     * of 12^3 126 -> 114 us.  With variable mass, which reads every line three times, the copy is
-     * faster (146 us against 160 us, 447 states) */
+     * read from global memory (L2, L1) in rounds instead of from a staged copy.  Step of 3000 states,
+     * global / staged, FP64 and all-FP32: 8^3 0.254 / 0.255 and 0.218 / 0.224 ms, 12^3 0.583 / 0.634
+     * and 0.473 / 0.527, 16^3 1.83 / 2.02 and 1.13 / 1.21.  With variable mass, which reads every line
+     * three times, the copy is faster (pass A of 447 states of 12^3 146 us against 160 us) */
     static constexpr bool from_global = circ && CG::dims == 3 && !VAR;
     static constexpr int threads = !circ ? (G::ntot >= 512 ? 512 : pts)
                                  : CG::nmax > 32 ? (lines < 128 ? 128 : lines > 256 ? 256 : lines)

@@ -1,6 +1,13 @@
 /*
  * The stream path: one TD half step on 3D lattices whose state does not fit one CTA (32^3,
- * 48^3, ...) and whose axes have at most 64 points (longer axes: wtd_path3d.cuh).
+ * 48^3, ...), whose axes have at most 64 points and whose plane and column blocks fit shared memory
+ * (StreamFit in wtd_api.cuh: all such lattices with constant mass or in the FP32-mixed forms; with
+ * variable mass in FP64 a (y, z) plane of up to 64 x 62 points, 64 x 64 is 512 bytes too large).
+ *
+ * Against the staged path in FP64, ms per step: 64^3 constant mass 200 states 17.0 / 20.6 (lines of 64
+ * points spill in the density and x kernels, 4.7, 1.0 and 0.4 KB a thread, and still win); 50x54x64
+ * 300 states 15.5 / 22.1, 10 states 1.02 / 2.71; 48^3 601 states 13.5 / 25.1; 32^3 variable mass 1500
+ * states 14.0 / 29.3.  64^3 variable mass in FP64 stays on the staged path (200 states: 42.5).
  *
  * Every derivative is a folded circulant product of one real lattice line in one thread's
  * registers (wtd_circ.cuh), so a half step is a chain of plain streaming kernels:

@@ -100,7 +100,9 @@ def test_stream_path_takes_more_than_65535_states(has_gpu):
 def test_densities_are_those_of_the_returned_states(has_gpu, name, nwf, prec):
     """the complex64 forms sum the densities of the states that the call leaves, not of states rounded
     once more afterwards: rho and nu formed from the returned states agree to FP64 rounding of sums of
-    nwf terms"""
+    nwf terms.  And the returned states are normalised: rounding the 4 N reals of a state once each
+    (2^-25 rms / sqrt 3 relative and independent) leaves its norm off by 2^-24 / sqrt(4 N) or less,
+    2e-9 is five times that at the smallest N; a state scaled after it was rounded keeps up to 3e-8"""
     from wslda_b200 import TDRun
     proj, d = inputs(name, nwf)
     N = proj.numel
@@ -111,6 +113,7 @@ def test_densities_are_those_of_the_returned_states(has_gpu, name, nwf, prec):
         y, dens = r.states().reshape(2, nwf, N), r.densities()
         f = np.asarray(d["occ"])[:, None]
         u, v = y[0], y[1]
+        assert np.abs((np.abs(y) ** 2).sum(axis=(0, 2)) * proj.dv - 1.0).max() < 2e-9
         nu = ((u * v.conj()) * (1.0 - 2.0 * f) * 0.5).sum(0)
         got = dens[:2 * N].view(np.complex128)
         # relative to sum |u v|, which the signed sum nu cancels from

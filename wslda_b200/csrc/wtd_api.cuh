@@ -54,7 +54,8 @@ struct wtd_ctx {
     int p1grid;                 /* CTAs of the plane H kernel */
     /* stream path (wtd_stream3d.cuh) */
     int stream;
-    double *sc, *part;          /* scale 1/norm of every state; partial sums of <H> and the norm */
+    double *sc, *scn, *part;    /* scale 1/norm of every state, and of the corrector at the end of a call;
+                                 * partial sums of <H> and the norm */
     int xgrid;                  /* CTAs of the x kernel */
     int gpt, gpl, gx;           /* state chunks of the point, plane and x density kernels */
     void *xfer;                 /* bounded staging buffer of the mixed-precision uploads/downloads */
@@ -647,9 +648,9 @@ template <typename TY, typename TH, typename TC> struct Stream {
     }
     template <int PASS> static int abm(wtd_ctx *c, const StepArgs &a)
     {
-        k3s_abm<TY, TH, TC, WTD_NHIST, PASS><<<S3::states_grid(c->S), S3::AT, 0, c->st>>>(a, (const C *)c->kbuf, c->sc, c->part);
+        k3s_abm<TY, TH, TC, WTD_NHIST, PASS><<<S3::states_grid(c->S), S3::AT, 0, c->st>>>(a, (const C *)c->kbuf, c->sc, c->scn, c->part);
         WTD_LAUNCHED(c);
-        return PASS == 3 ? WTD_OK : sum(c, 2 * S3::ACH, c->sc, 1);
+        return PASS == 3 || PASS == 5 ? WTD_OK : sum(c, 2 * S3::ACH, PASS == 4 ? c->scn : c->sc, 1);
     }
     static int attrs()
     {
@@ -678,9 +679,15 @@ template <typename TY, typename TH, typename TC> struct Stream {
             WTD_LAUNCHED(c);
             WTD_TRY(sum(c, 2 * S3::NQB, c->qpe, 0));
         }
-        WTD_TRY(p == 0 ? abm<0>(c, a) : p == 1 ? abm<1>(c, a) : p == 2 ? abm<2>(c, a) : abm<3>(c, a));
-        if (p == 3) return WTD_OK;
-        if (final) WTD_TRY(rescale(c));
+        if (p == 1 && final && sizeof(TY) < sizeof(double2)) {
+            WTD_TRY(abm<4>(c, a));
+            WTD_TRY(abm<5>(c, a));
+            WTD_TRY(scale_one(c));
+        } else {
+            WTD_TRY(p == 0 ? abm<0>(c, a) : p == 1 ? abm<1>(c, a) : p == 2 ? abm<2>(c, a) : abm<3>(c, a));
+            if (p == 3) return WTD_OK;
+            if (final) WTD_TRY(rescale(c));
+        }
         return dens(c, c->wcnt, grad);
     }
     /* density sums of the current states with per-state weights w */
@@ -702,6 +709,10 @@ template <typename TY, typename TH, typename TC> struct Stream {
     {
         k3s_rescale<TY><<<S3::states_grid(c->S), S3::AT, 0, c->st>>>((TY *)c->y, c->sc, c->S);
         WTD_LAUNCHED(c);
+        return scale_one(c);
+    }
+    static int scale_one(wtd_ctx *c)
+    {
         k3s_fill<<<(c->S + 255) / 256, 256, 0, c->st>>>(c->sc, 1.0, c->S);
         WTD_LAUNCHED(c);
         return WTD_OK;
@@ -1267,7 +1278,7 @@ size_t wtd_device_bytes(int nwf, int precision)
         if (precision != WTD_FP64) b += n2 * sizeof(double2);
     } else if (path != PATH_FUSED)
         b += n2 * (precision == WTD_FP64 ? sizeof(double2) : sizeof(float2));
-    if (path == PATH_STREAM) b += (S + stream_part_words(nwf)) * sizeof(double);
+    if (path == PATH_STREAM) b += (2 * S + stream_part_words(nwf)) * sizeof(double);
     return b;
 }
 
@@ -1361,6 +1372,7 @@ int wtd_create(wtd_ctx **out, int nwf, int precision, int device)
     }
     if (c->stream) {
         ALLOC(c->sc, nwf * sizeof(double));
+        ALLOC(c->scn, nwf * sizeof(double));
         ALLOC(c->part, stream_part_words(nwf) * sizeof(double));
     }
     if (c->staged) {
@@ -1419,7 +1431,7 @@ int wtd_destroy(wtd_ctx *c)
                 for (int i = 0; i < 4096; i++) cudaEventDestroy(c->ev[p][k][i]);
     void *ptrs[] = {c->y, c->cf, c->occ, c->kp2, c->wcnt, c->dslot, c->qpe, c->dens, c->pots, c->qfld, c->dqf, c->ework,
                     c->eout, c->tw, c->ktab, c->stage, c->extra, c->ddx, c->ddy, c->ddz, c->dlap, c->dalap, c->stage3d,
-                    c->kbuf, c->xfer, c->sc, c->part};
+                    c->kbuf, c->xfer, c->sc, c->scn, c->part};
     for (size_t i = 0; i < sizeof(ptrs) / sizeof(ptrs[0]); i++) if (ptrs[i]) cudaFree(ptrs[i]);
     for (int h = 0; h < WTD_NHIST; h++) if (c->hist[h]) cudaFree(c->hist[h]);
     if (c->st) cudaStreamDestroy(c->st);

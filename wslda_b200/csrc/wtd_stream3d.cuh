@@ -24,9 +24,9 @@
  * The updated states are stored before their norm is known.  What is formed from them next is
  * linear in the state (h) or quadratic (<H>, densities), so those kernels work on the stored values
  * and the state's scale 1/norm (k3s_sum) is taken in FP64 where the result is next used or summed.
- * In the last half step of a call the states are scaled in place (k3s_rescale) before their
- * densities are summed, which are then those of the states that the caller sees.  Precision forms
- * as in the fused pass: TY storage of the states, TH of the ABM history, TC of the derivatives;
+ * The last half step of a call leaves normalised states, whose densities are summed from what is
+ * stored: in FP64 scaled in place (k3s_rescale), in the complex64 forms stored after a pass for the
+ * norm (k3s_abm, PASS 4 and 5).  Precision forms as in the fused pass: TY storage of the states, TH of the ABM history, TC of the derivatives;
  * local terms, ABM sums, norms, <H> and density sums are FP64.
  */
 #ifndef WTD_STREAM3D_CUH
@@ -336,12 +336,18 @@ __global__ void __launch_bounds__(128) k3s_sum(const double *part, int np, int S
 }
 
 /* the ABM update of one chunk of one component of one state, y and h times the state's scale.  PASS 0:
- * f_k = h - E y (or read from ring slot NH-1), predictor into y, partial corrector P; 1: corrector into y; 2: norm only;
- * 3: f_k only */
+ * f_k = h - E y (or read from ring slot NH-1), predictor into y, partial corrector P; 1: corrector
+ * into y; 2: norm only; 3: f_k only; 4: norm of the corrector, nothing stored; 5: corrector times the
+ * scale scn of its norm into y.  4 and 5 end a call in the complex64 forms: the normalised value is
+ * rounded once.  Scaling the rounded corrector in place would leave it as it is where the scale is
+ * closer to 1 than half a unit of FP32, and with it a norm off by up to 3e-8 (48^3, 256 states, 20
+ * steps: density error 4.9e-8 against 3.3e-8) */
 template <typename TY, typename TH, typename TC, int NH, int PASS>
 __global__ void __launch_bounds__(S3::AT) k3s_abm(StepArgs a, const typename cplx<TC>::t *__restrict__ H,
-                                                  const double *__restrict__ sc, double *__restrict__ npart)
+                                                  const double *__restrict__ sc, const double *__restrict__ scn,
+                                                  double *__restrict__ npart)
 {
+    constexpr bool CORR = PASS == 1 || PASS == 4 || PASS == 5;
     typedef typename cplx<TC>::t C;
     constexpr int N = S3::N, AT = S3::AT, AE = S3::AE;
     __shared__ double red[80];
@@ -349,9 +355,9 @@ __global__ void __launch_bounds__(S3::AT) k3s_abm(StepArgs a, const typename cpl
     if (n >= a.S) return;
     const size_t fb = ((size_t)comp * a.S + n) * N;
     const int i0 = ch * (AT * AE) + threadIdx.x;
-    const bool haveH = PASS == 1 || PASS == 3 || (PASS == 0 && !a.fk_given);
+    const bool haveH = CORR || PASS == 3 || (PASS == 0 && !a.fk_given);
     TY *Y = (TY *)a.y;
-    constexpr int NR = PASS == 0 ? NH - 1 : PASS == 1 ? 1 : 0;
+    constexpr int NR = PASS == 0 ? NH - 1 : CORR ? 1 : 0;
     TY yv[AE];
     C hv[AE];
     TH fr[AE][NR > 0 ? NR : 1], fkg[AE];
@@ -365,12 +371,12 @@ __global__ void __launch_bounds__(S3::AT) k3s_abm(StepArgs a, const typename cpl
 #pragma unroll
                 for (int j = 0; j < NR; j++) fr[k][j] = ld_stream((const TH *)a.slot[j] + fb + i);
                 if (!haveH) fkg[k] = ld_stream((const TH *)a.slot[NH - 1] + fb + i);
-            } else if (PASS == 1) {
+            } else if (CORR) {
                 fr[k][0] = ld_stream((const TH *)a.slot[NH - 2] + fb + i);
             }
         }
     }
-    const double s = sc[n], E = haveH ? a.qpe[n] : 0.0, dt = a.dt;
+    const double s = sc[n], E = haveH ? a.qpe[n] : 0.0, dt = a.dt, sn = PASS == 5 ? scn[n] : 1.0;
     double nrm = 0.0;
 #pragma unroll
     for (int k = 0; k < AE; k++) {
@@ -403,15 +409,19 @@ __global__ void __launch_bounds__(S3::AT) k3s_abm(StepArgs a, const typename cpl
             const double2 P = make_double2(y0.x + dt * sa.y, y0.y - dt * sa.x);
             if (haveH) st_stream((TH *)a.slot[NH - 1] + fb + i, from_d<TH>(fk));
             st_stream((TH *)a.slot[NH - 2] + fb + i, from_d<TH>(P));
-        } else if (PASS == 1) {
+        } else if (CORR) {
             const double2 P = to_d(fr[k][0]);
             out.x = dt * fk.y * Abm<NH>::c + P.x;
             out.y = -dt * fk.x * Abm<NH>::c + P.y;
         }
+        if (PASS == 5) {
+            Y[fb + i] = from_d<TY>(make_double2(out.x * sn, out.y * sn));
+            continue;
+        }
         nrm += out.x * out.x + out.y * out.y;
-        if (PASS != 2) Y[fb + i] = from_d<TY>(out);
+        if (PASS != 2 && PASS != 4) Y[fb + i] = from_d<TY>(out);
     }
-    if (PASS != 3) {
+    if (PASS != 3 && PASS != 5) {
         nrm = block_sum(nrm, red);
         if (threadIdx.x == 0) npart[(size_t)n * (2 * S3::ACH) + comp * S3::ACH + ch] = nrm;
     }

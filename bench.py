@@ -623,7 +623,7 @@ def adjoint_c4(args, dev):
 
 def probe(args):
     """one form of one workload on one GPU: device time of --steps steps after the initial
-    measurement and --warmup steps (the case the ncu captures of the line path run)"""
+    measurement and --warmup steps (the case the ncu captures run)"""
     import torch
     from wslda_b200 import TDRun
     wl = C5 if args.workload == "c5" else WORKLOADS[args.workload]

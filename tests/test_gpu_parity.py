@@ -106,9 +106,17 @@ def test_t3d_wide_axes_to_64(has_gpu, nwf):
 
 
 @pytest.mark.gpu
-def test_t3d_wide_h32(has_gpu):
-    """the same lattice in the all-FP32 form"""
-    _track_fp64("t3d_wide", 4, 2, 1e-5)
+def test_t3d_wide_variable_mass(has_gpu):
+    """the same range with variable mass in FP64 (64 x 52 x 60, ASLDA), where the plane's and the column
+    block's arrays nearly fill shared memory"""
+    _compare("t3d_wide_var", nwf=7, nsteps=2, nmeas=1)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("name,nwf", [("t3d_wide", 4), ("t3d_wide_var", 7)])
+def test_t3d_wide_h32(has_gpu, name, nwf):
+    """the same lattices in the all-FP32 form"""
+    _track_fp64(name, nwf, 2, 1e-5)
 
 
 @pytest.mark.gpu
